@@ -208,8 +208,8 @@ GH_EMU_HD bool inv_cube_rn(double s, double& out) {
   return inv_cube_core(E, (bits & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull, out);
 }
 
-// s^(-3/2) within about half an ulp (not correctly rounded: the tree walk's FP64
-// interactions, which sum in their own order anyway); false outside [2^-577, 2^602).
+// s^(-3/2) of a rounded s within about half an ulp (not correctly rounded; the tree walk
+// takes mass_inv_cube below, which starts from the differences); false outside [2^-577, 2^602).
 GH_EMU_HD bool rsqrt_cube(double s, double& out) {
   const uint64_t bits = dbits(s);
   const int E = (int)(bits >> 52);
@@ -386,6 +386,126 @@ GH_EMU_HD bool pair_inv_cube_rn(double dx, double dy, double dz, int eps2_E, uin
     M = M2;
   }
   return inv_cube_core(E, M, out);
+}
+
+// ---------------------------------------------------------------------------
+// m s^(-3/2) with s = dx^2 + dy^2 + dz^2 + eps^2, all in 64-bit fixed point and rounded
+// once (the tree walk's FP64 interactions): the differences are aligned at the largest
+// exponent e (|d| 2^(62-e) as integers), squared to their top 64 bits and summed, so
+// s = S 2^(2e-60) with S to about 2^-58 of s and an exponent that is even as the root
+// wants it; one residual h = 1 - n y0^2 of the FP32 seed, |h| < 2^-20, then
+// s^(-3/2) = y0^3 (1 + 3/2 h + 15/8 h^2), whose first omitted term is below 2^-58.
+
+GH_EMU_HD int clz64(uint64_t v) {
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)v);
+#else
+  return __builtin_clzll(v);
+#endif
+}
+
+// v >> s, 0 for s > 63.
+GH_EMU_HD uint64_t shr_clamp(uint64_t v, int s) {
+#ifdef __CUDA_ARCH__
+  uint64_t r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+  return r;
+#else
+  return s > 63 ? 0 : v >> s;
+#endif
+}
+
+// a b / 2^64, short by at most 2 (the low halves' product and two carries are left out).
+GH_EMU_HD uint64_t umulhi_low(uint64_t a, uint64_t b) {
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  return (uint64_t)ah * bh + (((uint64_t)ah * bl) >> 32) + (((uint64_t)al * bh) >> 32);
+}
+
+// The same for signed b, a < 2^63.
+GH_EMU_HD int64_t smulhi_low(uint64_t a, int64_t b) {
+  const int32_t ah = (int32_t)(a >> 32), bh = (int32_t)(b >> 32);
+  const uint32_t al = (uint32_t)a, bl = (uint32_t)b;
+  return (int64_t)ah * bh + (int64_t)(((uint64_t)(uint32_t)ah * bl) >> 32) + (((int64_t)al * bh) >> 32);
+}
+
+// Top 64 bits of x^2, short by at most 2.
+GH_EMU_HD uint64_t square_hi(uint64_t x) {
+  const uint32_t h = (uint32_t)(x >> 32), l = (uint32_t)x;
+  return (uint64_t)h * h + 2 * (((uint64_t)h * l) >> 32);
+}
+
+// eps^2 for the aligned sum: eps^2 = W 2^(2(Ee-1023)-60), W in [2^60, 2^62); W = 0 for
+// eps^2 = 0.  False (the caller keeps to FP64) outside [2^-300, 2^300].
+GH_EMU_HD bool align_eps2(double eps2, int& Ee, uint64_t& W) {
+  const uint64_t b = dbits(eps2);
+  const int E = (int)(b >> 52);
+  Ee = 0;
+  W = 0;
+  if (b == 0) return true;
+  if ((unsigned)(E - 723) > 600u) return false;
+  const int e = E - 1023, half = e >> 1;  // floor(e / 2)
+  Ee = half + 1023;
+  W = ((b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << (8 + (e & 1));
+  return true;
+}
+
+// s = n 4^e, n = N10 2^-62 in [1, 4); false unless the largest of |dx|, |dy|, |dz|, eps
+// lies in [2^-150, 2^151).
+GH_EMU_HD bool aligned_norm2(double dx, double dy, double dz, int Ee, uint64_t W, uint64_t& N10, int& e) {
+  const uint64_t M52 = 0x000FFFFFFFFFFFFFull, ONE = 0x0010000000000000ull;
+  const uint64_t bx = dbits(dx), by = dbits(dy), bz = dbits(dz);
+  const int Ex = (int)(bx >> 52) & 0x7FF, Ey = (int)(by >> 52) & 0x7FF, Ez = (int)(bz >> 52) & 0x7FF;
+  int E = Ex > Ey ? Ex : Ey;
+  E = Ez > E ? Ez : E;
+  E = Ee > E ? Ee : E;
+  // a zero or subnormal difference has its implicit bit set here, 2^-800 below the rest
+  const uint64_t X = shr_clamp(((bx & M52) | ONE) << 10, E - Ex);
+  const uint64_t Y = shr_clamp(((by & M52) | ONE) << 10, E - Ey);
+  const uint64_t Z = shr_clamp(((bz & M52) | ONE) << 10, E - Ez);
+  const uint64_t S = square_hi(X) + square_hi(Y) + square_hi(Z) + shr_clamp(W, 2 * (E - Ee));  // [2^60, 2^64)
+  const int big = (S >> 62) != 0;
+  N10 = big ? S : S << 2;
+  e = E - 1023 + big;
+  return (unsigned)(E - 873) <= 300u;
+}
+
+// Seed of 1/sqrt(n) as Y0 = y0 2^30 in (2^29, 2^30] to rounding, and the residual h = 1 - n y0^2 as
+// H = h 2^60; false unless |h| < 2^-20.
+GH_EMU_HD bool rsqrt_seed_residual(uint64_t N10, uint32_t& Y0, uint64_t& Y0sq, int64_t& H) {
+  const uint32_t hi = (uint32_t)(N10 >> 32), odd = hi >> 31;  // hi in [2^30, 2^32)
+  const float nf = bitsf((hi >> (7 + odd)) + ((126u + odd) << 23));
+  // y0 in (1/2, 1] plus 1 leaves y0 2^23 in the significand (no conversion instruction)
+  Y0 = (fbits(rsqrt_seed(nf) + 1.0f) - 0x3F800000u) << 7;
+  Y0sq = (uint64_t)Y0 * Y0;  // y0^2 2^60, at most a little above 2^60
+  H = (int64_t)((1ull << 60) - umulhi_low(N10, Y0sq << 2));
+  return (uint64_t)(H + (1ll << 40)) < (1ull << 41);
+}
+
+GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
+  uint64_t N10, Y0sq;
+  uint32_t Y0;
+  int64_t H;
+  int e;
+  const uint64_t bm = dbits(m);
+  const int Em = (int)(bm >> 52) & 0x7FF;
+  bool ok = aligned_norm2(dx, dy, dz, Ee, W, N10, e);
+  ok &= (unsigned)(Em - 523) <= 1000u;  // |m| in [2^-500, 2^501)
+  ok &= rsqrt_seed_residual(N10, Y0, Y0sq, H);
+  if (!ok) return false;
+  // y0^3 2^61, then times 1 + c, c = h (3/2 + 15/8 h) as C = c 2^60, |C| < 2^41
+  const uint64_t Y3 = umulhi_low(Y0sq << 2, (uint64_t)Y0 << 33);
+  const int32_t h = (int32_t)(H >> 10);  // h 2^50
+  const int64_t C = H + (H >> 1) + ((((int64_t)h * h >> 20) * 15) >> 23);
+  const uint64_t F = Y3 + (uint64_t)(smulhi_low(Y3, C << 22) >> 18);
+  // times the mass's significand mm in [1, 2): T0 = mm y^3 2^62 in [2^59, 2^63]
+  const uint64_t T0 = umulhi_low(F << 2, ((bm & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 11);
+  const int lz = clz64(T0);
+  const uint64_t T = T0 << lz;
+  const uint64_t mant = (T >> 11) + ((T >> 10) & 1);  // in [2^52, 2^53]
+  // s^(-3/2) = y^3 2^(-3e): out = mant 2^k
+  const int k = (Em - 1023) - 51 - lz - 3 * e;
+  out = bitsd((((uint64_t)(k + 1074) << 52) + mant) | (bm & 0x8000000000000000ull));
+  return true;
 }
 
 }  // namespace emu

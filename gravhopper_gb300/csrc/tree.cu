@@ -752,25 +752,38 @@ constexpr int TW_FQ = 32;
 constexpr int TW_FQ_ROUND = 28;
 static_assert((TW_FQ & (TW_FQ - 1)) == 0, "the FIFO index wraps with a mask");
 
-// One FP64 interaction: the cell's monopole (nM) with s^(-3/2) on the integer pipes,
-// FP64 Newton steps outside the emulation's range.
+// Softening as the fixed-point interaction wants it (f64emu.cuh); ok = false keeps every
+// interaction on the FP64 operations. 
+struct WalkEps {
+  double eps2;
+  uint64_t W;
+  int E;
+  bool ok;
+};
+
+// One FP64 interaction: the cell's monopole (nM) times s^(-3/2), from the differences to
+// the rounded factor in 64-bit fixed point; FP64 operations outside that form's range.
+// Bound by the FP64 pipe, which a warp's DFMA holds for 17 cycles of the SM and a DADD
+// or DMUL for 20 (measured): three differences and three sums are left on it, 111 of the
+// 106-cycle round at N = 1M (idle lanes are skipped), where s and its factor took four
+// more.  The fixed-point part is about 190 integer instructions (issue 58 % busy).
+// Force at N = 1M Hernquist + disk: theta 0.7 29.0 -> 18.5 ms, theta 0.5 71.6 -> 44.9;
+// the differences as FMAs by an opaque 1.0 (17 cycles instead of 20): 18.8.
 template <bool GUARD>
 __device__ __forceinline__ void walk_interact_f64(const dvec4* __restrict__ nM, int node, double p0, double p1,
-                                                  double p2, double eps2, double& ax, double& ay, double& az) {
+                                                  double p2, const WalkEps& E, double& ax, double& ay, double& az) {
   const dvec4 M = nM[node];
   const double dx = M.x - p0, dy = M.y - p1, dz = M.z - p2;
-  const double s = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-  if (!GUARD || s != 0.0) {
-    double y3;
-    if (!emu::rsqrt_cube(s, y3)) {
-      const double y = rsqrt_f64(s);
-      y3 = y * (y * y);
-    }
-    const double f = M.w * y3;
-    ax = fma(f, dx, ax);
-    ay = fma(f, dy, ay);
-    az = fma(f, dz, az);
+  double f;
+  if (!(E.ok && emu::mass_inv_cube(M.w, dx, dy, dz, E.E, E.W, f))) {
+    const double s = fma(dx, dx, fma(dy, dy, fma(dz, dz, E.eps2)));
+    if (GUARD && s == 0.0) return;
+    const double y = rsqrt_f64(s);
+    f = M.w * (y * (y * y));
   }
+  ax = fma(f, dx, ax);
+  ay = fma(f, dy, ay);
+  az = fma(f, dz, az);
 }
 
 template <bool GUARD, bool MIXED, bool STATS, class Epi>
@@ -788,9 +801,15 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     p1 = tpos[3 * t + 1];
     p2 = tpos[3 * t + 2];
   }
-  const float h0 = (float)p0, h1 = (float)p1, h2 = (float)p2;
-  const float l0 = f32_lo(p0, h0), l1 = f32_lo(p1, h1), l2 = f32_lo(p2, h2);
-  const f2 h01 = f2make(h0, h1), l01 = f2make(l0, l1);
+  const float h0 = (float)p0, h1 = (float)p1;
+  float h2 = (float)p2;
+  float l2 = f32_lo(p2, h2);
+  const f2 h01 = f2make(h0, h1);
+  f2 l01 = f2make(f32_lo(p0, h0), f32_lo(p1, h1));
+  // FP64: keeps the compiler from forming the residuals again inside the loop to save
+  // registers, where each is three FP64-pipe instructions (one residual per interaction
+  // was: 29.0 against 18.5 ms per force at N = 1M, theta 0.7)
+  if (!MIXED) asm volatile("" : "+f"(h2), "+f"(l2), "+l"(l01));
   // d^2 below this needs the exact test: FP32 differences lose too much relative to
   // |x|, and FP32 stays in its normal range (with theta >= 1e-3 a cell whose size^2
   // is below that range is then accepted, as the exact test would)
@@ -802,6 +821,9 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
   int pending = 0;
   __shared__ int fq[MIXED ? 1 : TW_FQ][TW_THREADS];  // FP64: this lane's accepted cells, FIFO
   int fq_head = 0, fq_n = 0;
+  WalkEps we;
+  we.eps2 = eps2;
+  we.ok = emu::align_eps2(eps2, we.E, we.W);
   unsigned n_step = 0, n_visit = 0, n_inter = 0, n_exact = 0, n_leaf = 0, n_chain = 0;  // walk counters (STATS)
   int skip = valid ? 0 : 0x7fffffff;
   int node = __reduce_min_sync(0xffffffffu, skip);
@@ -881,7 +903,7 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
           const int c = fq[fq_head][threadIdx.x];
           fq_head = (fq_head + 1) & (TW_FQ - 1);
           fq_n--;
-          walk_interact_f64<GUARD>(nM, c, p0, p1, p2, eps2, ax, ay, az);
+          walk_interact_f64<GUARD>(nM, c, p0, p1, p2, we, ax, ay, az);
         }
       }
     }
@@ -908,7 +930,7 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
       const int c = fq[fq_head][threadIdx.x];
       fq_head = (fq_head + 1) & (TW_FQ - 1);
       fq_n--;
-      walk_interact_f64<GUARD>(nM, c, p0, p1, p2, eps2, ax, ay, az);
+      walk_interact_f64<GUARD>(nM, c, p0, p1, p2, we, ax, ay, az);
     }
   }
   if (STATS) {

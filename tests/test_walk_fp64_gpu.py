@@ -1,0 +1,35 @@
+"""The FP64 tree walk where its interaction changes form: scales inside and outside the
+fixed-point factor's range, with and without softening, against the oracle tree.
+Tolerance as for every FP64 tree force: rms <= 1e-12, max <= 1e-9 per particle."""
+import numpy as np
+import pytest
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def check(got, ref):
+    num, den = np.linalg.norm(got - ref, axis=1), np.linalg.norm(ref, axis=1)
+    assert np.all(num[den == 0] == 0)
+    r = num[den > 0] / den[den > 0]
+    assert float(np.sqrt(np.mean(r * r))) <= 1e-12 and r.max() <= 1e-9, (np.sqrt(np.mean(r * r)), r.max())
+
+
+# 1e-50, 1e44: differences below 2^-150 and near 2^147, where some pairs leave the range
+@pytest.mark.parametrize("scale", [1e-50, 1e-45, 1e-3, 1.0, 1e44])
+@pytest.mark.parametrize("eps", [0.0, 0.05])
+def test_scales(lib, cuda, scale, eps):
+    from gravhopper_gb300 import _jbgrav, ics
+    ic = ics.plummer(700, b=1.0, totmass=1.0, seed=4)
+    pos = ic["pos"] * scale
+    got = _jbgrav.tree_force(pos, ic["mass"], eps * scale, 0.6)
+    check(got * scale * scale, oracle.tree_force(pos, ic["mass"], eps * scale, 0.6) * scale * scale)
+
+
+def test_signs_and_sizes_of_masses(lib, cuda):
+    from gravhopper_gb300 import _jbgrav, ics
+    ic = ics.plummer(500, b=1.0, totmass=1.0, seed=5)
+    rng = np.random.default_rng(6)
+    mass = ic["mass"] * 10.0 ** rng.uniform(-170, 150, 500)  # beyond 2^+-500 at both ends
+    check(_jbgrav.tree_force(ic["pos"], mass, 0.05, 0.0), oracle.tree_force(ic["pos"], mass, 0.05, 0.0))
