@@ -738,10 +738,10 @@ __device__ __forceinline__ double rsqrt_f64(double s) {
   return y;
 }
 
-// MIXED: accepted cells interact in FP32: the hi/lo split offset of the cell's
+// Mixed: accepted cells interact in FP32: the hi/lo split offset of the cell's
 // centre (keeps ~2^-48 of |x|) plus the FP32 offset of its centre of mass; partial
 // sums folded into a two-sum (hi, lo) accumulator every 32 interactions.  Otherwise
-// FP64 with s^(-3/2) from the integer-pipe reciprocal square root (f64emu.cuh).
+// FP64 with the factor from fixed point (f64emu.cuh).
 // The opening decisions are the same exact ones in both forms.
 constexpr int TW_FOLD = 32;
 // FP64: a lane's accepted cells wait in a FIFO of TW_FQ entries and are evaluated in
@@ -786,10 +786,81 @@ __device__ __forceinline__ void walk_interact_f64(const dvec4* __restrict__ nM, 
   az = fma(f, dz, az);
 }
 
-template <bool GUARD, bool MIXED, bool STATS, class Epi>
+// A target's position as the opening test wants it: FP32 hi and residual, and the
+// squared distance below which the exact test is needed (FP32 differences lose too much
+// relative to |x|, and FP32 stays in its normal range: with theta >= 1e-3 a cell whose
+// size^2 is below that range is then accepted, as the exact test would).
+struct WalkTarget {
+  f2 h01, l01;
+  float h2, l2, near2;
+};
+__device__ __forceinline__ WalkTarget walk_target(double p0, double p1, double p2) {
+  WalkTarget T;
+  const float h0 = (float)p0, h1 = (float)p1;
+  T.h2 = (float)p2;
+  T.l2 = f32_lo(p2, T.h2);
+  T.h01 = f2make(h0, h1);
+  T.l01 = f2make(f32_lo(p0, h0), f32_lo(p1, h1));
+  T.near2 = fmaxf(1e-18f * (h0 * h0 + h1 * h1 + T.h2 * T.h2), 1e-30f);
+  return T;
+}
+
+// Offset of a cell's centre (A, Lo: its record) from the target.
+__device__ __forceinline__ void walk_offset(const WalkTarget& T, const float4& A, const float4& Lo, f2& dxy, float& dz) {
+  dxy = f2add(f2sub(f2make(A.x, A.y), T.h01), f2sub(f2make(Lo.x, Lo.y), T.l01));
+  dz = (A.z - T.h2) + (Lo.z - T.l2);
+}
+
+// The opening test of an internal cell: accepted when size / distance < theta, decided in
+// FP32 outside the margins, else with the reference's FP64 operations (exact counts those).
+__device__ __forceinline__ bool walk_accept(const WalkTarget& T, f2 dxy, float dz, float s2, float th2_lo, float th2_hi,
+                                            const dvec4* __restrict__ nC, int node, double p0, double p1, double p2,
+                                            double theta, unsigned& exact) {
+  float dx, dy;
+  f2split(dxy, dx, dy);
+  const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+  // d2 = inf (overflow) accepts, as the exact test does for so distant a cell
+  const bool usable = d2 > T.near2;
+  if (usable && s2 < th2_lo * d2) return true;
+  if (usable && s2 > th2_hi * d2) return false;
+  // gravoct_calc_accel opening test with the reference's FP64 operations
+  exact++;
+  const dvec4 C = nC[node];
+  const double e0 = dsub(C.x, p0), e1 = dsub(C.y, p1), e2 = dsub(C.z, p2);
+  double nd = dmul(e0, e0);
+  nd = dadd(nd, dmul(e1, e1));
+  nd = dadd(nd, dmul(e2, e2));
+  return ddiv(C.w, dsqrt(nd)) < theta;
+}
+
+// Walk counters of a warp into stats.
+__device__ __forceinline__ void walk_count(unsigned long long* stats, unsigned n_step, unsigned n_visit, unsigned n_inter,
+                                           unsigned n_exact, unsigned n_leaf, unsigned n_chain) {
+  // one cell record read per warp step; the other counts summed over lanes
+  n_visit = __reduce_add_sync(0xffffffffu, n_visit);
+  n_inter = __reduce_add_sync(0xffffffffu, n_inter);
+  n_exact = __reduce_add_sync(0xffffffffu, n_exact);
+  n_leaf = __reduce_add_sync(0xffffffffu, n_leaf);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&stats[0], (unsigned long long)n_step);
+    atomicAdd(&stats[1], (unsigned long long)n_visit);
+    atomicAdd(&stats[2], (unsigned long long)n_inter);
+    atomicAdd(&stats[3], (unsigned long long)n_exact);
+    atomicAdd(&stats[4], (unsigned long long)n_leaf);
+    atomicAdd(&stats[5], (unsigned long long)n_chain);
+  }
+}
+
+// A cell with one child cell: the child's subtree ends where the cell's does.
+__device__ __forceinline__ bool walk_is_chain(const WalkRec* __restrict__ nR, int node, int nnodes) {
+  const int nxt = __float_as_int(nR[node].L.w);
+  return nxt != node + 1 && node + 1 < nnodes && __float_as_int(nR[node + 1].L.w) == nxt;
+}
+
+template <bool GUARD, bool STATS, class Epi>
 __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
-    tree_walk_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, const dvec4* __restrict__ nM,
-                     int nnodes, const double* __restrict__ tpos, const uint32_t* __restrict__ order, int64_t nt,
+    tree_walk_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, int nnodes,
+                     const double* __restrict__ tpos, const uint32_t* __restrict__ order, int64_t nt,
                      double eps2, double theta, float th2_lo, float th2_hi, Epi epi,
                      unsigned long long* __restrict__ stats) {
   const int64_t slot = (int64_t)blockIdx.x * TW_THREADS + threadIdx.x;
@@ -801,115 +872,55 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     p1 = tpos[3 * t + 1];
     p2 = tpos[3 * t + 2];
   }
-  const float h0 = (float)p0, h1 = (float)p1;
-  float h2 = (float)p2;
-  float l2 = f32_lo(p2, h2);
-  const f2 h01 = f2make(h0, h1);
-  f2 l01 = f2make(f32_lo(p0, h0), f32_lo(p1, h1));
-  // FP64: keeps the compiler from forming the residuals again inside the loop to save
-  // registers, where each is three FP64-pipe instructions (one residual per interaction
-  // was: 29.0 against 18.5 ms per force at N = 1M, theta 0.7)
-  if (!MIXED) asm volatile("" : "+f"(h2), "+f"(l2), "+l"(l01));
-  // d^2 below this needs the exact test: FP32 differences lose too much relative to
-  // |x|, and FP32 stays in its normal range (with theta >= 1e-3 a cell whose size^2
-  // is below that range is then accepted, as the exact test would)
-  const float near2 = fmaxf(1e-18f * (h0 * h0 + h1 * h1 + h2 * h2), 1e-30f);
+  const WalkTarget T = walk_target(p0, p1, p2);
   const float eps2f = (float)eps2;
-  double ax = 0.0, ay = 0.0, az = 0.0;
-  float px = 0.f, py = 0.f, pz = 0.f;            // FP32 partial (MIXED)
+  float px = 0.f, py = 0.f, pz = 0.f;                                // FP32 partial
   float hx = 0.f, hy = 0.f, hz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;  // two-sum hi, lo
   int pending = 0;
-  __shared__ int fq[MIXED ? 1 : TW_FQ][TW_THREADS];  // FP64: this lane's accepted cells, FIFO
-  int fq_head = 0, fq_n = 0;
-  WalkEps we;
-  we.eps2 = eps2;
-  we.ok = emu::align_eps2(eps2, we.E, we.W);
   unsigned n_step = 0, n_visit = 0, n_inter = 0, n_exact = 0, n_leaf = 0, n_chain = 0;  // walk counters (STATS)
   int skip = valid ? 0 : 0x7fffffff;
   int node = __reduce_min_sync(0xffffffffu, skip);
   while (node < nnodes) {
     if (STATS) {
       n_step++;
-      // a cell with one child cell: the child's subtree ends where the cell's does
-      const int nxt = __float_as_int(nR[node].L.w);
-      if (nxt != node + 1 && node + 1 < nnodes && __float_as_int(nR[node + 1].L.w) == nxt) n_chain++;
+      n_chain += walk_is_chain(nR, node, nnodes);
     }
     int lane_next = skip;
     if (node >= skip) {
       if (STATS) n_visit++;
       const float4 A = nR[node].A;
       const float4 Lo = nR[node].L;
-      float4 O;  // loaded with the rest of the record: most visits are accepted
-      if (MIXED) O = nR[node].O;
+      const float4 O = nR[node].O;  // loaded with the rest of the record: most visits are accepted
       const int nx = __float_as_int(Lo.w);
       bool accept = (nx == node + 1);  // leaf
-      // (x, y) offsets as one f32x2 pair, z alone
-      const f2 dxy = f2add(f2sub(f2make(A.x, A.y), h01), f2sub(f2make(Lo.x, Lo.y), l01));
-      const float dz = (A.z - h2) + (Lo.z - l2);
-      float dx, dy;
-      f2split(dxy, dx, dy);
-      if (!accept) {
-        const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        const float s2 = A.w;
-        // d2 = inf (overflow) accepts, as the exact test does for so distant a cell
-        const bool usable = d2 > near2;
-        if (usable && s2 < th2_lo * d2) {
-          accept = true;
-        } else if (usable && s2 > th2_hi * d2) {
-          accept = false;
-        } else {
-          // gravoct_calc_accel opening test with the reference's FP64 operations
-          if (STATS) n_exact++;
-          const dvec4 C = nC[node];
-          const double e0 = dsub(C.x, p0), e1 = dsub(C.y, p1), e2 = dsub(C.z, p2);
-          double nd = dmul(e0, e0);
-          nd = dadd(nd, dmul(e1, e1));
-          nd = dadd(nd, dmul(e2, e2));
-          accept = ddiv(C.w, dsqrt(nd)) < theta;
-        }
-      }
+      f2 dxy;
+      float dz;
+      walk_offset(T, A, Lo, dxy, dz);
+      if (!accept) accept = walk_accept(T, dxy, dz, A.w, th2_lo, th2_hi, nC, node, p0, p1, p2, theta, n_exact);
       if (accept) {
         if (STATS) {
           n_inter++;
           if (nx == node + 1) n_leaf++;
         }
-        if (MIXED) {
-          float ex, ey;
-          f2split(f2add(dxy, f2make(O.x, O.y)), ex, ey);
-          const float ez = dz + O.z;
-          const float s = fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, eps2f)));
-          float r = rsqrt_approx(s);
-          if (GUARD) r = s > 0.f ? r : 0.f;
-          const float f = O.w * (r * (r * r));
-          px = fmaf(f, ex, px);
-          py = fmaf(f, ey, py);
-          pz = fmaf(f, ez, pz);
-        } else {
-          fq[(fq_head + fq_n) & (TW_FQ - 1)][threadIdx.x] = node;  // evaluated in a later round
-          fq_n++;
-        }
+        float ex, ey;
+        f2split(f2add(dxy, f2make(O.x, O.y)), ex, ey);
+        const float ez = dz + O.z;
+        const float s = fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, eps2f)));
+        float r = rsqrt_approx(s);
+        if (GUARD) r = s > 0.f ? r : 0.f;
+        const float f = O.w * (r * (r * r));
+        px = fmaf(f, ex, px);
+        py = fmaf(f, ey, py);
+        pz = fmaf(f, ez, pz);
         skip = nx;
         lane_next = nx;
       } else {
         lane_next = node + 1;
       }
     }
-    if (!MIXED) {
-      // a round of FP64 interactions when enough lanes have one waiting; a FIFO that
-      // just became full forces one, so a FIFO never holds more than TW_FQ
-      const unsigned waiting = __ballot_sync(0xffffffffu, fq_n > 0);
-      if (__popc(waiting) >= TW_FQ_ROUND || __any_sync(0xffffffffu, fq_n == TW_FQ)) {
-        if (fq_n > 0) {
-          const int c = fq[fq_head][threadIdx.x];
-          fq_head = (fq_head + 1) & (TW_FQ - 1);
-          fq_n--;
-          walk_interact_f64<GUARD>(nM, c, p0, p1, p2, we, ax, ay, az);
-        }
-      }
-    }
     // fold the FP32 partials every TW_FOLD warp steps (at most one interaction per
     // target per step): a warp-uniform branch
-    if (MIXED && ++pending == TW_FOLD) {
+    if (++pending == TW_FOLD) {
       float sx, ex;
       two_sum(hx, px, sx, ex);
       hx = sx;
@@ -925,33 +936,192 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     }
     node = __reduce_min_sync(0xffffffffu, lane_next);
   }
-  if (!MIXED) {
-    while (fq_n > 0) {  // the cells still waiting, in order
-      const int c = fq[fq_head][threadIdx.x];
-      fq_head = (fq_head + 1) & (TW_FQ - 1);
-      fq_n--;
-      walk_interact_f64<GUARD>(nM, c, p0, p1, p2, we, ax, ay, az);
-    }
+  if (STATS) walk_count(stats, n_step, n_visit, n_inter, n_exact, n_leaf, n_chain);
+  if (valid)
+    epi(t, (double)hx + (double)qx + (double)px, (double)hy + (double)qy + (double)py,
+        (double)hz + (double)qz + (double)pz);
+}
+
+// How a walk is split over warps: `segs` warps per 32 targets, each walking one range of
+// the preorder.  Targets that have a place of their own in it (particles, sorted points)
+// visit about as many cells in each doubling of the distance from that place, so the
+// ranges grow geometrically with it; 32 unsorted points are anywhere, so theirs are equal.
+struct WalkSplit {
+  int segs;
+  double* part;           // [group][seg][component][lane] partial sums
+  int* count;             // per group: segments finished (zero between launches)
+  const int* base;        // first node of each key-ordered particle (null: equal ranges)
+  const uint64_t* keys;   // the particles' first two key words, n each,
+  const uint64_t* tkeys;  // and the sorted points' (null: the targets are the particles)
+  int64_t n;
+};
+constexpr float TW_SEG_NEAR = 128.f;  // nodes around its own place that a group visits densely
+
+// Place in the preorder of target slot q.
+__device__ __forceinline__ int walk_own(const WalkSplit& sp, int64_t q, int64_t nt, int nnodes) {
+  if (!sp.tkeys) return sp.base[q];
+  const uint64_t k0 = sp.tkeys[q], k1 = sp.tkeys[nt + q];
+  int64_t a = 0, b = sp.n;  // first particle whose key is not below the point's
+  while (a < b) {
+    const int64_t m = (a + b) >> 1;
+    const uint64_t w = sp.keys[m];
+    if (w < k0 || (w == k0 && sp.keys[sp.n + m] < k1))
+      a = m + 1;
+    else
+      b = m;
   }
-  if (STATS) {
-    // one cell record read per warp step; the other counts summed over lanes
-    n_visit = __reduce_add_sync(0xffffffffu, n_visit);
-    n_inter = __reduce_add_sync(0xffffffffu, n_inter);
-    n_exact = __reduce_add_sync(0xffffffffu, n_exact);
-    n_leaf = __reduce_add_sync(0xffffffffu, n_leaf);
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(&stats[0], (unsigned long long)n_step);
-      atomicAdd(&stats[1], (unsigned long long)n_visit);
-      atomicAdd(&stats[2], (unsigned long long)n_inter);
-      atomicAdd(&stats[3], (unsigned long long)n_exact);
-      atomicAdd(&stats[4], (unsigned long long)n_leaf);
-      atomicAdd(&stats[5], (unsigned long long)n_chain);
-    }
+  return a < sp.n ? sp.base[a] : nnodes;
+}
+
+// First node of segment s (of K) for a group whose own place is node `own` (-1: none).
+__device__ __forceinline__ int walk_bound(int s, int K, int own, int nnodes) {
+  if (s <= 0) return 0;
+  if (s >= K) return nnodes;
+  if (own < 0) return (int)((int64_t)nnodes * s / K);
+  const float left = log2f(1.f + (float)own / TW_SEG_NEAR), right = log2f(1.f + (float)(nnodes - own) / TW_SEG_NEAR);
+  const float u = (left + right) * (float)s / (float)K;
+  const float d = TW_SEG_NEAR * (exp2f(fabsf(u - left)) - 1.f);
+  const int b = u < left ? own - (int)d : own + (int)d;
+  return b < 0 ? 0 : (b > nnodes ? nnodes : b);
+}
+
+// FP64 walk.  SPLIT: warp w of the grid takes segment w % segs of target group w / segs.
+// The segment's first node a lies inside a chain of ancestor cells; the warp first takes
+// each lane's decisions on that chain (their interactions belong to the segments that hold
+// those cells), so that every cell and interaction is met exactly once, in the segment that
+// holds it.  The group's last segment to finish adds the partial sums in segment order: the
+// result does not depend on timing.
+template <bool GUARD, bool STATS, bool SPLIT, class Epi>
+__global__ void __launch_bounds__(TW_THREADS, TW_MINB)
+    tree_walk_f64_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, const dvec4* __restrict__ nM,
+                         int nnodes, const double* __restrict__ tpos, const uint32_t* __restrict__ order, int64_t nt,
+                         double eps2, double theta, float th2_lo, float th2_hi, Epi epi, WalkSplit sp,
+                         unsigned long long* __restrict__ stats) {
+  const int lane = threadIdx.x & 31;
+  const unsigned set = SPLIT ? blockIdx.x / sp.segs : blockIdx.x;  // of neighbouring target groups
+  const int seg = SPLIT ? (int)(blockIdx.x - set * sp.segs) : 0;
+  const int64_t group = (int64_t)set * (TW_THREADS / 32) + (threadIdx.x >> 5);
+  if (group * 32 >= nt) return;  // whole warps
+  const int64_t slot = group * 32 + lane;
+  const bool valid = slot < nt;
+  const int64_t t = valid ? (order ? (int64_t)order[slot] : slot) : 0;
+  double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+  if (valid) {
+    p0 = tpos[3 * t];
+    p1 = tpos[3 * t + 1];
+    p2 = tpos[3 * t + 2];
   }
-  if (MIXED) {
-    ax = (double)hx + (double)qx + (double)px;
-    ay = (double)hy + (double)qy + (double)py;
-    az = (double)hz + (double)qz + (double)pz;
+  WalkTarget T = walk_target(p0, p1, p2);
+  // keeps the compiler from forming the residuals again inside the loop to save registers,
+  // where each is three FP64-pipe instructions (one residual per interaction was: 29.0
+  // against 18.5 ms per force at N = 1M, theta 0.7)
+  asm volatile("" : "+f"(T.h2), "+f"(T.l2), "+l"(T.l01));
+  double ax = 0.0, ay = 0.0, az = 0.0;
+  __shared__ int fq[TW_FQ][TW_THREADS];  // this lane's accepted cells, FIFO
+  int fq_head = 0, fq_n = 0;
+  WalkEps we;
+  we.eps2 = eps2;
+  we.ok = emu::align_eps2(eps2, we.E, we.W);
+  unsigned n_step = 0, n_visit = 0, n_inter = 0, n_exact = 0, n_leaf = 0, n_chain = 0;  // walk counters (STATS)
+  int skip = valid ? 0 : 0x7fffffff;
+  int end = nnodes;
+  if (SPLIT) {
+    const int64_t mid = group * 32 + 16 < nt ? group * 32 + 16 : nt - 1;
+    const int own = sp.base ? walk_own(sp, mid, nt, nnodes) : -1;
+    const int first = walk_bound(seg, sp.segs, own, nnodes);
+    end = walk_bound(seg + 1, sp.segs, own, nnodes);
+    int c = 0;
+    while (c < first) {  // the cells that hold `first`
+      const float4 Lo = nR[c].L;
+      const int nx = __float_as_int(Lo.w);
+      if (nx <= first) {
+        c = nx;
+        continue;
+      }
+      if (c >= skip) {
+        f2 dxy;
+        float dz;
+        const float4 A = nR[c].A;
+        walk_offset(T, A, Lo, dxy, dz);
+        if (walk_accept(T, dxy, dz, A.w, th2_lo, th2_hi, nC, c, p0, p1, p2, theta, n_exact)) skip = nx;
+      }
+      c++;
+    }
+    if (skip < first) skip = first;
+  }
+  int node = __reduce_min_sync(0xffffffffu, skip);
+  while (node < end) {
+    if (STATS) {
+      n_step++;
+      n_chain += walk_is_chain(nR, node, nnodes);
+    }
+    int lane_next = skip;
+    if (node >= skip) {
+      if (STATS) n_visit++;
+      const float4 A = nR[node].A;
+      const float4 Lo = nR[node].L;
+      const int nx = __float_as_int(Lo.w);
+      bool accept = (nx == node + 1);  // leaf
+      if (!accept) {
+        f2 dxy;
+        float dz;
+        walk_offset(T, A, Lo, dxy, dz);
+        accept = walk_accept(T, dxy, dz, A.w, th2_lo, th2_hi, nC, node, p0, p1, p2, theta, n_exact);
+      }
+      if (accept) {
+        if (STATS) {
+          n_inter++;
+          if (nx == node + 1) n_leaf++;
+        }
+        fq[(fq_head + fq_n) & (TW_FQ - 1)][threadIdx.x] = node;  // evaluated in a later round
+        fq_n++;
+        skip = nx;
+        lane_next = nx;
+      } else {
+        lane_next = node + 1;
+      }
+    }
+    // a round of FP64 interactions when enough lanes have one waiting; a FIFO that
+    // just became full forces one, so a FIFO never holds more than TW_FQ
+    const unsigned waiting = __ballot_sync(0xffffffffu, fq_n > 0);
+    if (__popc(waiting) >= TW_FQ_ROUND || __any_sync(0xffffffffu, fq_n == TW_FQ)) {
+      if (fq_n > 0) {
+        const int c = fq[fq_head][threadIdx.x];
+        fq_head = (fq_head + 1) & (TW_FQ - 1);
+        fq_n--;
+        walk_interact_f64<GUARD>(nM, c, p0, p1, p2, we, ax, ay, az);
+      }
+    }
+    node = __reduce_min_sync(0xffffffffu, lane_next);
+  }
+  while (fq_n > 0) {  // the cells still waiting, in order
+    const int c = fq[fq_head][threadIdx.x];
+    fq_head = (fq_head + 1) & (TW_FQ - 1);
+    fq_n--;
+    walk_interact_f64<GUARD>(nM, c, p0, p1, p2, we, ax, ay, az);
+  }
+  if (STATS) walk_count(stats, n_step, n_visit, n_inter, n_exact, n_leaf, n_chain);
+  if (SPLIT) {
+    __syncwarp();
+    double* mine = sp.part + (group * sp.segs + seg) * 96 + lane;
+    mine[0] = ax;
+    mine[32] = ay;
+    mine[64] = az;
+    __threadfence();
+    __syncwarp();
+    int last = 0;
+    if (lane == 0) last = atomicAdd(&sp.count[group], 1) == sp.segs - 1;
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (!last) return;
+    __threadfence();
+    const double* all = sp.part + group * sp.segs * 96 + lane;
+    ax = ay = az = 0.0;
+    for (int k = 0; k < sp.segs; k++) {
+      ax += __ldcg(all + 96 * k);
+      ay += __ldcg(all + 96 * k + 32);
+      az += __ldcg(all + 96 * k + 64);
+    }
+    if (lane == 0) sp.count[group] = 0;  // ready for the next launch
   }
   if (valid) epi(t, ax, ay, az);
 }
@@ -962,6 +1132,8 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
 struct TreeWS {
   Buffer part, root, keys, keys_tmp, idx, idx_tmp, rs, lp, cnt, depth, base, scan, flags;
   Buffer nA, nC, nM, fxl, fxt, xh[2];
+  Buffer wpart, wcount;       // split walks: partial sums, finished segments per group
+  size_t wcount_zeroed = 0;
   Buffer tkeys, tkeys_tmp, tidx, tidx_tmp, trs;  // target points' walk order
   Buffer list;                // particle lists: key fallbacks, then cell openers
   Buffer cells;               // (internal cell, opener) pairs
@@ -981,6 +1153,7 @@ static NodeArrays node_arrays(TreeWS& ws) {
 }
 
 struct BuiltTree {
+  int64_t n = 0;  // particles
   int nnodes = 0;
   int maxdepth = 0;
   const uint32_t* torder = nullptr;  // target points in key order (when sorted)
@@ -1142,6 +1315,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
       GH_LAUNCH_CHECK();
     }
   }
+  out->n = n;
   out->nnodes = nnodes;
   out->maxdepth = maxdepth;
   return GH_OK;
@@ -1154,21 +1328,91 @@ static bool g_stats_on = false;
 static int64_t g_stats_walks = 0;
 static Buffer g_stats[64];
 
-template <bool G, bool MX, class Epi>
-static void launch_walk(const NodeArrays& na, const BuiltTree& bt, const double* tpos, const uint32_t* order,
-                        int64_t nt, double eps2, double theta, float lo, float hi, const Epi& epi,
-                        unsigned long long* stats, cudaStream_t st) {
-  const unsigned blocks = (unsigned)((nt + TW_THREADS - 1) / TW_THREADS);
+// Warps per target group of an FP64 walk.  A warp walks hundreds to thousands of cells in
+// a chain of dependent steps, so a walk with fewer groups than the GPU holds warps
+// (36 per SM) takes as long as its longest chain; splitting the chains fills the GPU, at
+// about 2 % more steps per doubling (the ancestors of each segment's first cell).
+// Up to 1024 groups some 28,000 warps in all were fastest, at most 64 per group (256 for
+// unsorted points, whose walks have no dense part); above, three warps per group below
+// 2048 groups, two up to 12,288 (3/4 of the machine's warps and more were slower split
+// further).  Force, unsplit -> split, theta 0.7: N = 2000 Plummer 770 -> 314 us, 8000
+// 1001 -> 486; Hernquist + disk 16,384 1376 -> 707, 60,013 1945 -> 1421, 131,072 2698 ->
+// 2618, 262,144 4978 -> 4716; at 1,048,576 two warps would cost 18.7 -> 19.1 ms.  Points
+// in a 250,000-particle system, theta 0.5: 100 unsorted 17.6 -> 0.9 ms, 8100 17.9 -> 3.0,
+// 30,011 sorted 6.4 -> 3.6.
+static int walk_segments(int64_t groups, bool placed) {
+  if (groups > 12288) return 1;
+  if (groups >= 2048) return 2;
+  if (groups > 1024) return 3;
+  const int64_t cap = placed ? 64 : 256, k = 28672 / groups;
+  return (int)(k < cap ? k : cap);
+}
+
+template <bool G, class Epi>
+static int launch_walk_f64(TreeWS& ws, const NodeArrays& na, const BuiltTree& bt, const double* tpos,
+                           const uint32_t* order, int64_t nt, bool self, double eps2, double theta, float lo, float hi,
+                           const Epi& epi, unsigned long long* stats, cudaStream_t st) {
+  const int64_t groups = (nt + 31) / 32;
+  WalkSplit sp = {};
+  sp.segs = stats ? 1 : walk_segments(groups, self || order);  // the counters are those of whole walks
+  const size_t cb = (size_t)groups * sizeof(int);
+  if (sp.segs > 1) {  // at most 22 MB of scratch; without it the walk is not split
+    int rc = ensure(ws.wpart, (size_t)groups * sp.segs * 96 * sizeof(double));
+    if (rc == GH_OK && ws.wcount.bytes < cb) ws.wcount_zeroed = 0;
+    if (rc == GH_OK) rc = ensure(ws.wcount, cb);
+    if (rc == GH_ERR_OOM) {
+      clear_error();
+      sp.segs = 1;
+    } else if (rc != GH_OK) {
+      return rc;
+    }
+  }
+  const unsigned blocks = (unsigned)((groups + TW_THREADS / 32 - 1) / (TW_THREADS / 32)) * (unsigned)sp.segs;
+  if (sp.segs > 1) {
+    if (ws.wcount_zeroed < cb) {
+      GH_CUDA_TRY(cudaMemsetAsync(ws.wcount.ptr, 0, ws.wcount.bytes, st));
+      ws.wcount_zeroed = ws.wcount.bytes;
+    }
+    sp.part = (double*)ws.wpart.ptr;
+    sp.count = (int*)ws.wcount.ptr;
+    if (self || order) sp.base = (const int*)ws.base.ptr;
+    if (!self && order) {
+      sp.keys = (const uint64_t*)ws.keys.ptr;
+      sp.tkeys = (const uint64_t*)ws.tkeys.ptr;
+      sp.n = bt.n;
+    }
+  }
+  prof_begin(st);
   if (stats)
-    tree_walk_kernel<G, MX, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nnodes, tpos, order, nt,
-                                                                      eps2, theta, lo, hi, epi, stats);
+    tree_walk_f64_kernel<G, true, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nnodes, tpos, order,
+                                                                             nt, eps2, theta, lo, hi, epi, sp, stats);
+  else if (sp.segs > 1)
+    tree_walk_f64_kernel<G, false, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nnodes, tpos, order,
+                                                                             nt, eps2, theta, lo, hi, epi, sp, nullptr);
   else
-    tree_walk_kernel<G, MX, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nnodes, tpos, order,
-                                                                       nt, eps2, theta, lo, hi, epi, nullptr);
+    tree_walk_f64_kernel<G, false, false, Epi><<<blocks, TW_THREADS, 0, st>>>(
+        na.R, na.C, na.M, bt.nnodes, tpos, order, nt, eps2, theta, lo, hi, epi, sp, nullptr);
+  prof_end(st);
+  return GH_OK;
+}
+
+template <bool G, class Epi>
+static void launch_walk_mixed(const NodeArrays& na, const BuiltTree& bt, const double* tpos, const uint32_t* order,
+                              int64_t nt, double eps2, double theta, float lo, float hi, const Epi& epi,
+                              unsigned long long* stats, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((nt + TW_THREADS - 1) / TW_THREADS);
+  prof_begin(st);
+  if (stats)
+    tree_walk_kernel<G, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, bt.nnodes, tpos, order, nt, eps2, theta,
+                                                                  lo, hi, epi, stats);
+  else
+    tree_walk_kernel<G, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, bt.nnodes, tpos, order, nt, eps2, theta,
+                                                                   lo, hi, epi, nullptr);
+  prof_end(st);
 }
 
 template <class Epi>
-static int tree_walk(TreeWS& ws, const BuiltTree& bt, const double* tpos, const uint32_t* order, int64_t nt,
+static int tree_walk(TreeWS& ws, const BuiltTree& bt, const double* tpos, const uint32_t* order, int64_t nt, bool self,
                      double eps, double theta, int precision, const Epi& epi, cudaStream_t st) {
   if (nt == 0) return GH_OK;
   Trace tr("tree walk");
@@ -1197,19 +1441,17 @@ static int tree_walk(TreeWS& ws, const BuiltTree& bt, const double* tpos, const 
     stats = (unsigned long long*)b.ptr;
     g_stats_walks++;
   }
-  prof_begin(st);
   if (mixed) {
     if (guard)
-      launch_walk<true, true>(na, bt, tpos, order, nt, eps2, theta, lo, hi, epi, stats, st);
+      launch_walk_mixed<true>(na, bt, tpos, order, nt, eps2, theta, lo, hi, epi, stats, st);
     else
-      launch_walk<false, true>(na, bt, tpos, order, nt, eps2, theta, lo, hi, epi, stats, st);
+      launch_walk_mixed<false>(na, bt, tpos, order, nt, eps2, theta, lo, hi, epi, stats, st);
   } else {
     if (guard)
-      launch_walk<true, false>(na, bt, tpos, order, nt, eps2, theta, lo, hi, epi, stats, st);
+      GH_TRY(launch_walk_f64<true>(ws, na, bt, tpos, order, nt, self, eps2, theta, lo, hi, epi, stats, st));
     else
-      launch_walk<false, false>(na, bt, tpos, order, nt, eps2, theta, lo, hi, epi, stats, st);
+      GH_TRY(launch_walk_f64<false>(ws, na, bt, tpos, order, nt, self, eps2, theta, lo, hi, epi, stats, st));
   }
-  prof_end(st);
   GH_LAUNCH_CHECK();
   return GH_OK;
 }
@@ -1239,8 +1481,8 @@ int tree_force(const double* pos, const double* mass, int64_t np, const double* 
   BuiltTree bt;
   GH_TRY(tree_build(ws, pos, mass, np, eps, st, &bt, self ? nullptr : tpos, self ? 0 : nt));
   EpiStore epi{acc};
-  if (self) return tree_walk(ws, bt, pos, (const uint32_t*)ws.idx.ptr, np, eps, theta, precision, epi, st);
-  return tree_walk(ws, bt, tpos, bt.torder, nt, eps, theta, precision, epi, st);
+  if (self) return tree_walk(ws, bt, pos, (const uint32_t*)ws.idx.ptr, np, true, eps, theta, precision, epi, st);
+  return tree_walk(ws, bt, tpos, bt.torder, nt, false, eps, theta, precision, epi, st);
 }
 
 int tree_run(double* x, double* v, const double* mass, int64_t np, int64_t nsteps, double dt, double eps,
@@ -1273,7 +1515,7 @@ int tree_run(double* x, double* v, const double* mass, int64_t np, int64_t nstep
       epi.hist_x = hist_x + slot * np * 3;
       epi.hist_v = hist_v + slot * np * 3;
     }
-    GH_TRY(tree_walk(ws, bt, xh, (const uint32_t*)ws.idx.ptr, np, eps, theta, precision, epi, st));
+    GH_TRY(tree_walk(ws, bt, xh, (const uint32_t*)ws.idx.ptr, np, true, eps, theta, precision, epi, st));
   }
   return GH_OK;
 }
