@@ -481,6 +481,27 @@ GH_EMU_HD bool rsqrt_seed_residual(uint64_t N10, uint32_t& Y0, uint64_t& Y0sq, i
   return (uint64_t)(H + (1ll << 40)) < (1ull << 41);
 }
 
+// 1/sqrt(dx^2 + dy^2 + dz^2 + eps^2), rounded once (the potential's pairs); false outside
+// the range of aligned_norm2.
+GH_EMU_HD bool inv_distance(double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
+  uint64_t N10, Y0sq;
+  uint32_t Y0;
+  int64_t H;
+  int e;
+  bool ok = aligned_norm2(dx, dy, dz, Ee, W, N10, e);
+  ok &= rsqrt_seed_residual(N10, Y0, Y0sq, H);
+  if (!ok) return false;
+  // y 2^62 = y0 2^62 (1 + c), c = h (1/2 + 3/8 h) as C = c 2^60; the next term is below 2^-61
+  const int32_t h = (int32_t)(H >> 10);  // h 2^50
+  const int64_t C = (H >> 1) + ((((int64_t)h * h >> 20) * 3) >> 23);
+  const uint64_t y0 = (uint64_t)Y0 << 32;
+  const uint64_t Y = y0 + (uint64_t)(smulhi_low(y0, C << 22) >> 18);  // in [2^61, 2^62] to rounding
+  const int up = (int)(Y >> 62);
+  const uint64_t mant = (Y >> (9 + up)) + ((Y >> (8 + up)) & 1);  // in [2^52, 2^53]
+  out = bitsd(((uint64_t)(up - 53 - e + 1074) << 52) + mant);  // s^(-1/2) = y 2^-e
+  return true;
+}
+
 GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
   uint64_t N10, Y0sq;
   uint32_t Y0;
