@@ -51,6 +51,7 @@ struct TreeRoot {
   double c[3];
   double size;
   double inv;           // RN(1 / size)
+  float invf;
   long long margin;     // 0: fast keys allowed; -1: the FP64 recurrence for every particle
   int bad;              // a particle position or mass is NaN or infinite
   int lsb_m, lsb_f;     // fixed-point units (2^lsb) of the mass and first-moment sums
@@ -190,6 +191,7 @@ __global__ void root_kernel(const double* __restrict__ part, int nb, double eps,
     root->lsb_m = root->lsb_f = 0;
   }
   root->inv = ddiv(1.0, bs);
+  root->invf = (float)root->inv;
   root->margin = (bs > 0x1p-900 && bs < 0x1p+900 && amax < 0x1p+900) ? 0 : -1;
 }
 
@@ -225,70 +227,97 @@ __device__ __forceinline__ void warp_append(bool need, int64_t i, int* __restric
   if (need) list[base + __popc(mask & lane_mask_lt())] = (int)i;
 }
 
-// Fast keys where the decisions are provably the recurrence's (see root_kernel);
-// the other particles are listed for keys_exact_kernel, so that the FP64 recurrence
-// runs on full warps.
-__global__ void keys_kernel(const double* __restrict__ pos, int64_t n, const TreeRoot* __restrict__ root,
-                            int words, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx,
-                            int* __restrict__ list, int* __restrict__ count) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Fast keys where the decisions are provably the recurrence's (see root_kernel); the
+// block's other particles (about 2 %) then take the reference's recurrence
+// (gravoct_calc_subnode, _jbgrav.c:441-462), compacted so that it runs on full warps: it
+// is a chain of FP64 additions, each 20 cycles of the SM for a warp however many of its
+// lanes take part.  "p > c" is decided on the doubles' bits, in an order-preserving integer
+// form, which leaves the additions alone on the FP64 pipe (a DSETP costs as much as one).
+// N = 2000 26 -> 11 us, 60,013 39 -> 13, 1M 85 -> 58 against a fast-key kernel and a
+// recurrence kernel on a global list (52 us of the 85 were FP64-pipe comparisons, scalings
+// and conversions of the fast keys).  Blocks of 1024 from four blocks of 256 per SM on:
+// fewer, fuller warps in the chain.
+__device__ __forceinline__ int64_t ordered_bits(double x) {  // x is not -0.0
+  const int64_t b = __double_as_longlong(x);
+  return b ^ (int64_t)((uint64_t)(b >> 63) >> 1);
+}
+
+// floor(t 2^63) of t in (0, 1), 2^63 from 1 on, 0 for t <= 0: off the bits of t (its
+// comparisons, its scaling and its conversion would all be FP64-pipe instructions).
+__device__ __forceinline__ uint64_t unit_bits(double t) {
+  const int64_t b = __double_as_longlong(t);
+  if (b >= 0x3FF0000000000000ll) return 1ull << 63;
+  const uint64_t m = (((uint64_t)b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 10;
+  return b <= 0 ? 0ull : emu::shr_clamp(m, 1022 - (int)(b >> 52));
+}
+
+// |p| in FP32, short by less than 2^-20 of it (2^-126 for anything smaller, infinity
+// beyond the range).
+__device__ __forceinline__ float abs_f32(double p) {
+  const uint64_t b = (uint64_t)__double_as_longlong(p);
+  const int e = ((int)(b >> 52) & 0x7FF) - 896;
+  const float f = __uint_as_float(((uint32_t)e << 23) | ((uint32_t)(b >> 29) & 0x7FFFFFu));
+  return e <= 0 ? 0x1p-126f : (e >= 255 ? INFINITY : f);
+}
+
+template <int T>
+__global__ void __launch_bounds__(T)
+    keys_kernel(const double* __restrict__ pos, int64_t n, const TreeRoot* __restrict__ root, int words,
+                uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
+  __shared__ int list[T];
+  __shared__ int count;
+  __shared__ double offs[TREE_MAX_LEVELS];  // child-centre offsets 0.5 * halfsize = size 2^-(l+2), exact
+  const double S = root->size;
+  for (int l = threadIdx.x; l < words * KEY_LEVELS; l += T)
+    offs[l] = dmul(S, __longlong_as_double((long long)(1023 - (l + 2)) << 52));
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  const int64_t i = (int64_t)blockIdx.x * T + threadIdx.x;
   bool need = false;
   if (i < n) {
     idx[i] = (uint32_t)i;
     need = true;
     if (root->margin >= 0 && words == 2) {
-      uint64_t T[3];
+      uint64_t K[3];
       bool ok = true;
       const double inv = root->inv;
+      const float invf = root->invf;
 #pragma unroll
       for (int k = 0; k < 3; k++) {
         const double p = pos[3 * i + k];
-        const double t = fma(dsub(p, root->c[k]), inv, 0.5);
-        T[k] = t >= 1.0 ? (1ull << 63) : (t > 0.0 ? (uint64_t)(t * 0x1p63) : 0ull);
+        K[k] = unit_bits(fma(dsub(p, root->c[k]), inv, 0.5));
         // 2 * 2^63 * (E_c / size + 2^-52) + slack, in FP32 (a bound, not a value)
-        const float mf = fmaf(86016.f * 1.01f * fabsf((float)p), (float)inv, 5200.f);
-        const uint64_t r = T[k] & ((1ull << 21) - 1);
+        const float mf = fmaf(86016.f * 1.01f * abs_f32(p), invf, 5200.f);
+        const uint64_t r = K[k] & ((1ull << 21) - 1);
         ok = ok && mf < 1048576.f && r > (uint64_t)mf && r < (1ull << 21) - (uint64_t)mf;
       }
       if (ok) {
-        keys[i] = spread3(T[0] >> 42) | (spread3(T[1] >> 42) << 1) | (spread3(T[2] >> 42) << 2);
-        keys[n + i] = spread3(T[0] >> 21) | (spread3(T[1] >> 21) << 1) | (spread3(T[2] >> 21) << 2);
+        keys[i] = spread3(K[0] >> 42) | (spread3(K[1] >> 42) << 1) | (spread3(K[2] >> 42) << 2);
+        keys[n + i] = spread3(K[0] >> 21) | (spread3(K[1] >> 21) << 1) | (spread3(K[2] >> 21) << 2);
         need = false;
       }
     }
   }
-  warp_append(need, i, list, count);
-}
-
-// The reference's recurrence (gravoct_calc_subnode, _jbgrav.c:441-462) for the
-// listed particles.
-__global__ void keys_exact_kernel(const double* __restrict__ pos, int64_t n, const TreeRoot* __restrict__ root,
-                                  int words, uint64_t* __restrict__ keys, const int* __restrict__ list,
-                                  const int* __restrict__ count) {
-  // child-centre offsets 0.5 * halfsize = size 2^-(l+2), exact scalings of the root size
-  __shared__ double offs[TREE_MAX_LEVELS];
-  const double S = root->size;
-  for (int l = threadIdx.x; l < TREE_MAX_LEVELS; l += blockDim.x)
-    offs[l] = dmul(S, __longlong_as_double((long long)(1023 - (l + 2)) << 52));
+  warp_append(need, i, list, &count);
   __syncthreads();
-  const int cnt = *count;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += gridDim.x * blockDim.x) {
-    const int64_t i = list[q];
-    const double p0 = pos[3 * i], p1 = pos[3 * i + 1], p2 = pos[3 * i + 2];
-    double c0 = root->c[0], c1 = root->c[1], c2 = root->c[2];
-    for (int w = 0; w < words; w++) {
-      uint64_t k = 0;
+  if (threadIdx.x >= count) return;
+  const int64_t j = list[threadIdx.x];
+  // adding 0.0 turns -0.0 into 0.0; the sums below are never -0.0
+  const int64_t q0 = ordered_bits(dadd(pos[3 * j], 0.0)), q1 = ordered_bits(dadd(pos[3 * j + 1], 0.0)),
+                q2 = ordered_bits(dadd(pos[3 * j + 2], 0.0));
+  double c0 = dadd(root->c[0], 0.0), c1 = dadd(root->c[1], 0.0), c2 = dadd(root->c[2], 0.0);
+  for (int w = 0; w < words; w++) {
+    uint64_t k = 0;
 #pragma unroll 3
-      for (int l = 0; l < KEY_LEVELS; l++) {
-        const double off = offs[w * KEY_LEVELS + l];
-        const unsigned g0 = p0 > c0, g1 = p1 > c1, g2 = p2 > c2;
-        c0 = g0 ? dadd(c0, off) : dsub(c0, off);
-        c1 = g1 ? dadd(c1, off) : dsub(c1, off);
-        c2 = g2 ? dadd(c2, off) : dsub(c2, off);
-        k = (k << 3) | (uint64_t)(g0 | (g1 << 1) | (g2 << 2));
-      }
-      keys[(int64_t)w * n + i] = k;
+    for (int l = 0; l < KEY_LEVELS; l++) {
+      const double off = offs[w * KEY_LEVELS + l];
+      const unsigned g0 = q0 > ordered_bits(c0), g1 = q1 > ordered_bits(c1), g2 = q2 > ordered_bits(c2);
+      c0 = dadd(c0, g0 ? off : -off);
+      c1 = dadd(c1, g1 ? off : -off);
+      c2 = dadd(c2, g2 ? off : -off);
+      k = (k << 3) | (uint64_t)(g0 | (g1 << 1) | (g2 << 2));
     }
+    keys[(int64_t)w * n + j] = k;
   }
 }
 
@@ -1163,6 +1192,8 @@ struct BuiltTree {
 // cost exceeds what the coherent warps save).
 constexpr int64_t TGT_SORT_MIN = 8192;
 
+constexpr int64_t KEYS_WIDE = 4 * 152 * 256;
+
 static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t n, double eps,
                       cudaStream_t st, BuiltTree* out, const double* tpos = nullptr, int64_t nt = 0) {
   Trace tr("tree build");
@@ -1210,10 +1241,10 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
     uint32_t* itmp = (uint32_t*)ws.idx_tmp.ptr;
     int* flags = (int*)ws.flags.ptr;
     GH_CUDA_TRY(cudaMemsetAsync(flags, 0, 8 * sizeof(int), st));
-    keys_kernel<<<gn, T, 0, st>>>(pos, n, root, words, keys, idx, (int*)ws.list.ptr, flags + 3);
-    GH_LAUNCH_CHECK();
-    keys_exact_kernel<<<gn < 4 * 152 ? gn : 4 * 152, T, 0, st>>>(pos, n, root, words, keys, (const int*)ws.list.ptr,
-                                                                flags + 3);
+    if (n >= KEYS_WIDE)
+      keys_kernel<1024><<<(unsigned)((n + 1023) / 1024), 1024, 0, st>>>(pos, n, root, words, keys, idx);
+    else
+      keys_kernel<256><<<gn, 256, 0, st>>>(pos, n, root, words, keys, idx);
     GH_LAUNCH_CHECK();
     if (full_sort) {
       GH_TRY(radix_sort_keys(keys, idx, ktmp, itmp, words, KEY_BITS, n, (uint32_t*)ws.rs.ptr, st, flags + 5));
