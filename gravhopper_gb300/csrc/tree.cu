@@ -63,76 +63,101 @@ struct TreeRoot {
 constexpr int BB_THREADS = 256;
 constexpr int BB_BLOCKS = 304;
 
-// Per block: the box (min xyz, max xyz), whether any position or mass is not finite
-// (the reference's insert never terminates on such particles) and the largest |mass|,
-// 8 doubles.
-constexpr int BB_PART = 8;
+// Doubles ordered as integers (-0.0 below 0.0): comparisons of doubles would be FP64-pipe
+// instructions.
+__device__ __forceinline__ int64_t ordered_bits(double x) {
+  const int64_t b = __double_as_longlong(x);
+  return b ^ (int64_t)((uint64_t)(b >> 63) >> 1);
+}
+__device__ __forceinline__ double from_ordered(int64_t o) {
+  return __longlong_as_double(o ^ (int64_t)((uint64_t)(o >> 63) >> 1));
+}
+
+struct Box {
+  int64_t mn[3], mx[3];  // ordered_bits
+  int64_t m;             // bits of the largest |mass|
+  bool bad;              // a position or mass is not finite
+};
+
+__device__ __forceinline__ Box box_empty() {
+  Box b;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    b.mn[k] = 0x7FF0000000000000ll;               // +inf
+    b.mx[k] = 0x7FF0000000000000ll ^ -1ll;        // below every finite double
+  }
+  b.m = 0;
+  b.bad = false;
+  return b;
+}
+
+__device__ __forceinline__ void box_add(Box& b, const double* __restrict__ pos, const double* __restrict__ mass,
+                                        int64_t i) {
+  const int64_t mb = __double_as_longlong(mass[i]) & 0x7FFFFFFFFFFFFFFFll;
+  b.bad = b.bad || mb >= 0x7FF0000000000000ll;
+  b.m = mb > b.m ? mb : b.m;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double q = pos[3 * i + k];
+    b.bad = b.bad || (__double_as_longlong(q) & 0x7FF0000000000000ll) == 0x7FF0000000000000ll;
+    const int64_t o = ordered_bits(q);
+    b.mn[k] = o < b.mn[k] ? o : b.mn[k];
+    b.mx[k] = o > b.mx[k] ? o : b.mx[k];
+  }
+}
+
+__device__ __forceinline__ void box_merge(Box& a, const Box& b) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    a.mn[k] = b.mn[k] < a.mn[k] ? b.mn[k] : a.mn[k];
+    a.mx[k] = b.mx[k] > a.mx[k] ? b.mx[k] : a.mx[k];
+  }
+  a.m = b.m > a.m ? b.m : a.m;
+  a.bad = a.bad || b.bad;
+}
+
+// Merges the lanes' boxes; every lane gets the result.
+__device__ __forceinline__ void box_warp(Box& b) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    Box c;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      c.mn[k] = __shfl_xor_sync(0xffffffffu, b.mn[k], o);
+      c.mx[k] = __shfl_xor_sync(0xffffffffu, b.mx[k], o);
+    }
+    c.m = __shfl_xor_sync(0xffffffffu, b.m, o);
+    c.bad = false;
+    box_merge(b, c);
+  }
+  b.bad = __any_sync(0xffffffffu, b.bad);
+}
+
+// Merges a block's boxes (T threads); warp 0 gets the result.
+template <int T>
+__device__ __forceinline__ void box_block(Box& b) {
+  __shared__ Box part[T / 32];
+  box_warp(b);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    b = threadIdx.x < T / 32 ? part[threadIdx.x] : box_empty();
+    box_warp(b);
+  }
+}
 
 __global__ void __launch_bounds__(BB_THREADS)
     bbox_partial_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n,
-                        double* __restrict__ part) {
-  __shared__ double s_mn[3][BB_THREADS], s_mx[3][BB_THREADS];
-  __shared__ double s_m[BB_THREADS];
-  double mn[3], mx[3], mmax = 0.0;
-  bool have = false, bad = false;
-  for (int64_t i = (int64_t)blockIdx.x * BB_THREADS + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * BB_THREADS) {
-    const double mi = mass[i];
-    bad = bad || !isfinite(mi);
-    mmax = fmax(mmax, fabs(mi));
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      double q = pos[3 * i + k];
-      bad = bad || !isfinite(q);
-      if (!have) {
-        mn[k] = mx[k] = q;
-      } else {
-        if (q < mn[k]) mn[k] = q;
-        if (q > mx[k]) mx[k] = q;
-      }
-    }
-    have = true;
-  }
-  if (!have) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      mn[k] = __longlong_as_double(0x7ff0000000000000ll);   // +inf
-      mx[k] = __longlong_as_double(0xfff0000000000000ll);   // -inf
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    s_mn[k][threadIdx.x] = mn[k];
-    s_mx[k][threadIdx.x] = mx[k];
-  }
-  s_m[threadIdx.x] = mmax;
-  bad = __syncthreads_or(bad);
-  for (int s = BB_THREADS / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        double a = s_mn[k][threadIdx.x + s], b = s_mx[k][threadIdx.x + s];
-        if (a < s_mn[k][threadIdx.x]) s_mn[k][threadIdx.x] = a;
-        if (b > s_mx[k][threadIdx.x]) s_mx[k][threadIdx.x] = b;
-      }
-      s_m[threadIdx.x] = fmax(s_m[threadIdx.x], s_m[threadIdx.x + s]);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      part[BB_PART * blockIdx.x + k] = s_mn[k][0];
-      part[BB_PART * blockIdx.x + 3 + k] = s_mx[k][0];
-    }
-    part[BB_PART * blockIdx.x + 6] = bad ? 1.0 : 0.0;
-    part[BB_PART * blockIdx.x + 7] = s_m[0];
-  }
+                        Box* __restrict__ part) {
+  Box b = box_empty();
+  for (int64_t i = (int64_t)blockIdx.x * BB_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * BB_THREADS)
+    box_add(b, pos, mass, i);
+  box_block<BB_THREADS>(b);
+  if (threadIdx.x == 0) part[blockIdx.x] = b;
 }
 
 // treeforce_workhorse, _jbgrav.c:764-772: boxsize = extent_x + eps, replaced by
 // extent_i + eps when extent_i (without eps) exceeds it; centre = bbox midpoint.
-// One warp folds the per-block partial boxes.
 //
 // Fast keys.  The reference's cell centres follow c_{l+1} = RN(c_l +- size 2^-(l+2)).
 // Along a particle's own path the level-(l+1) centre lies within size 2^-(l+2) of p,
@@ -144,30 +169,14 @@ __global__ void __launch_bounds__(BB_THREADS)
 // E_c / size + 2^-52 of a multiple of 2^-42.  keys_kernel keeps that window, doubled,
 // in units of 2^-63; particles inside it take the reference's FP64 recurrence, as do
 // all particles when the box size is outside [2^-900, 2^900] (margin -1).
-__global__ void root_kernel(const double* __restrict__ part, int nb, double eps, TreeRoot* __restrict__ root) {
-  if (blockIdx.x) return;
-  const int lane = threadIdx.x;
-  const double inf = __longlong_as_double(0x7ff0000000000000ll);
-  double mn[3] = {inf, inf, inf}, mx[3] = {-inf, -inf, -inf}, mmax = 0.0;
-  bool bad = false;
-  for (int b = lane; b < nb; b += 32) {
-    for (int k = 0; k < 3; k++) {
-      const double a = part[BB_PART * b + k], c = part[BB_PART * b + 3 + k];
-      if (a < mn[k]) mn[k] = a;
-      if (c > mx[k]) mx[k] = c;
-    }
-    bad = bad || part[BB_PART * b + 6] != 0.0;
-    mmax = fmax(mmax, part[BB_PART * b + 7]);
+__device__ __forceinline__ void root_write(const Box& box, double eps, TreeRoot* __restrict__ root) {
+  double mn[3], mx[3];
+  for (int k = 0; k < 3; k++) {
+    mn[k] = from_ordered(box.mn[k]);
+    mx[k] = from_ordered(box.mx[k]);
   }
-  bad = __any_sync(0xffffffffu, bad);
-  for (int o = 16; o > 0; o >>= 1) mmax = fmax(mmax, __shfl_xor_sync(0xffffffffu, mmax, o));
-  for (int o = 16; o > 0; o >>= 1)
-    for (int k = 0; k < 3; k++) {
-      const double a = __shfl_xor_sync(0xffffffffu, mn[k], o), c = __shfl_xor_sync(0xffffffffu, mx[k], o);
-      if (a < mn[k]) mn[k] = a;
-      if (c > mx[k]) mx[k] = c;
-    }
-  if (lane) return;
+  const bool bad = box.bad;
+  const double mmax = __longlong_as_double(box.m);
   double bs = dadd(dsub(mx[0], mn[0]), eps);
   for (int k = 1; k < 3; k++)
     if (dsub(mx[k], mn[k]) > bs) bs = dadd(dsub(mx[k], mn[k]), eps);
@@ -193,6 +202,25 @@ __global__ void root_kernel(const double* __restrict__ part, int nb, double eps,
   root->inv = ddiv(1.0, bs);
   root->invf = (float)root->inv;
   root->margin = (bs > 0x1p-900 && bs < 0x1p+900 && amax < 0x1p+900) ? 0 : -1;
+}
+
+// One warp folds the per-block boxes.
+__global__ void root_kernel(const Box* __restrict__ part, int nb, double eps, TreeRoot* __restrict__ root) {
+  Box b = box_empty();
+  for (int k = threadIdx.x; k < nb; k += 32) box_merge(b, part[k]);
+  box_warp(b);
+  if (threadIdx.x == 0) root_write(b, eps, root);
+}
+
+// Both for a small system, in one block.
+constexpr int SB_THREADS = 1024;
+__global__ void __launch_bounds__(SB_THREADS)
+    box_root_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n, double eps,
+                    TreeRoot* __restrict__ root) {
+  Box b = box_empty();
+  for (int64_t i = threadIdx.x; i < n; i += SB_THREADS) box_add(b, pos, mass, i);
+  box_block<SB_THREADS>(b);
+  if (threadIdx.x == 0) root_write(b, eps, root);
 }
 
 // ---------------------------------------------------------------------------
@@ -237,10 +265,6 @@ __device__ __forceinline__ void warp_append(bool need, int64_t i, int* __restric
 // recurrence kernel on a global list (52 us of the 85 were FP64-pipe comparisons, scalings
 // and conversions of the fast keys).  Blocks of 1024 from four blocks of 256 per SM on:
 // fewer, fuller warps in the chain.
-__device__ __forceinline__ int64_t ordered_bits(double x) {  // x is not -0.0
-  const int64_t b = __double_as_longlong(x);
-  return b ^ (int64_t)((uint64_t)(b >> 63) >> 1);
-}
 
 // floor(t 2^63) of t in (0, 1), 2^63 from 1 on, 0 for t <= 0: off the bits of t (its
 // comparisons, its scaling and its conversion would all be FP64-pipe instructions).
@@ -302,7 +326,8 @@ __global__ void __launch_bounds__(T)
   __syncthreads();
   if (threadIdx.x >= count) return;
   const int64_t j = list[threadIdx.x];
-  // adding 0.0 turns -0.0 into 0.0; the sums below are never -0.0
+  // adding 0.0 turns -0.0, which ordered_bits puts below 0.0, into 0.0; the sums below
+  // are never -0.0
   const int64_t q0 = ordered_bits(dadd(pos[3 * j], 0.0)), q1 = ordered_bits(dadd(pos[3 * j + 1], 0.0)),
                 q2 = ordered_bits(dadd(pos[3 * j + 2], 0.0));
   double c0 = dadd(root->c[0], 0.0), c1 = dadd(root->c[1], 0.0), c2 = dadd(root->c[2], 0.0);
@@ -475,7 +500,9 @@ struct NodeArrays {
 struct FxMoments {
   fx::I192 c[4];
 };
-constexpr int MS_THREADS = 256, MS_ITEMS = 8, MS_TILE = MS_THREADS * MS_ITEMS;
+constexpr int MS_THREADS = 256, MS_ITEMS = 8, MS_TILE = MS_THREADS * MS_ITEMS, MS_BITS = 11;
+static_assert(MS_TILE == 1 << MS_BITS, "tiles are found by a shift");
+constexpr int SB_BITS = 8;  // small builds: tiles of one particle per thread
 
 __device__ __forceinline__ void fxm_add(FxMoments& a, const FxMoments& b) {
 #pragma unroll
@@ -492,9 +519,10 @@ __device__ __forceinline__ FxMoments fxm_zero() {
 // Prefix over the first j key-ordered particles (j <= n): the tile's prefix plus the
 // prefix within the tile.
 __device__ __forceinline__ FxMoments fxm_prefix(const FxMoments* __restrict__ local,
-                                                const FxMoments* __restrict__ tiles, int64_t j, int64_t n) {
-  if (j >= n) return tiles[(n + MS_TILE - 1) / MS_TILE];
-  FxMoments r = tiles[j / MS_TILE];
+                                                const FxMoments* __restrict__ tiles, int tile_bits, int64_t j,
+                                                int64_t n) {
+  if (j >= n) return tiles[((n - 1) >> tile_bits) + 1];
+  FxMoments r = tiles[j >> tile_bits];
   fxm_add(r, local[j]);
   return r;
 }
@@ -528,6 +556,46 @@ __device__ __forceinline__ int64_t cell_end(const uint64_t* __restrict__ keys, i
   return a + 1;
 }
 
+__device__ __forceinline__ double rcp_f64(double m);
+
+// Leaf k: its particle's position as its centre and centre of mass, and its mass.
+__device__ __forceinline__ void write_leaf(const NodeArrays& na, int k, int next, double x, double y, double z, double m) {
+  na.M[k] = make_dvec4(x, y, z, m);
+  const float hx = (float)x, hy = (float)y, hz = (float)z;
+  na.R[k].A = make_float4(hx, hy, hz, 0.f);
+  na.R[k].L = make_float4(f32_lo(x, hx), f32_lo(y, hy), f32_lo(z, hz), __int_as_float(next));
+  na.R[k].O = make_float4(0.f, 0.f, 0.f, (float)m);
+}
+
+// Internal cell k with centre and size C, holding the key-ordered particles [i, end): its
+// walk record and its monopole, from exact sums with one rounding each, then firstmoment /
+// mass (_jbgrav.c:478) with a Newton-refined reciprocal.
+__device__ __forceinline__ void write_cell(const NodeArrays& na, int k, int next, const dvec4& C, int64_t i, int64_t end,
+                                           int64_t n, int lsb_m, int lsb_f, const FxMoments* __restrict__ fx_local,
+                                           const FxMoments* __restrict__ fx_tiles, int tile_bits) {
+  const double c[3] = {C.x, C.y, C.z};
+  float4 A, Lo;
+  A.x = f32_hi(c[0]);
+  A.y = f32_hi(c[1]);
+  A.z = f32_hi(c[2]);
+  A.w = (float)dmul(C.w, C.w);
+  Lo.x = f32_lo(c[0], A.x);
+  Lo.y = f32_lo(c[1], A.y);
+  Lo.z = f32_lo(c[2], A.z);
+  Lo.w = __int_as_float(next);
+  na.R[k].A = A;
+  na.R[k].L = Lo;
+  const FxMoments Pi = fxm_prefix(fx_local, fx_tiles, tile_bits, i, n);
+  const FxMoments Pe = fxm_prefix(fx_local, fx_tiles, tile_bits, end, n);
+  const double cm = fx::to_double(fx::sub(Pe.c[0], Pi.c[0]), lsb_m);
+  const double r = rcp_f64(cm);
+  double com[3];
+#pragma unroll
+  for (int a2 = 0; a2 < 3; a2++) com[a2] = dmul(fx::to_double(fx::sub(Pe.c[a2 + 1], Pi.c[a2 + 1]), lsb_f), r);
+  na.M[k] = make_dvec4(com[0], com[1], com[2], cm);
+  na.R[k].O = make_float4((float)dsub(com[0], c[0]), (float)dsub(com[1], c[1]), (float)dsub(com[2], c[2]), (float)cm);
+}
+
 // Particle i opens the cells at levels lo = lp[i]+1 .. d (its leaf), nodes
 // base[i] .. base[i] + d - lo in preorder.  nodes_kernel writes the leaf: the
 // particle's position as its centre, its mass, its skip index (gravoct_finalize,
@@ -550,13 +618,7 @@ __global__ void nodes_kernel(int64_t n, const int* __restrict__ lp, const int* _
     const int k = base[i] + (d - lo);
     const int next = i + 1 < n ? base[i + 1] : nnodes;
     const int64_t p = perm[i];
-    const double m = mass[p];
-    const double x = pos[3 * p], y = pos[3 * p + 1], z = pos[3 * p + 2];
-    na.M[k] = make_dvec4(x, y, z, m);
-    const float hx = (float)x, hy = (float)y, hz = (float)z;
-    na.R[k].A = make_float4(hx, hy, hz, 0.f);
-    na.R[k].L = make_float4(f32_lo(x, hx), f32_lo(y, hy), f32_lo(z, hz), __int_as_float(next));
-    na.R[k].O = make_float4(0.f, 0.f, 0.f, (float)m);
+    write_leaf(na, k, next, pos[3 * p], pos[3 * p + 1], pos[3 * p + 2], mass[p]);
     need = d > lo;
     ncell = d - lo;
     k0 = base[i];
@@ -575,8 +637,6 @@ __global__ void nodes_kernel(int64_t n, const int* __restrict__ lp, const int* _
   first = __shfl_sync(0xffffffffu, first, 31) + incl - ncell;
   for (int j = 0; j < ncell; j++) cells[first + j] = make_int2(k0 + j, (int)i);
 }
-
-__device__ __forceinline__ double rcp_f64(double m);
 
 // Centres of the internal cells from the reference's FP64 recurrence along each
 // opener's digits (gravoct_add_particle, _jbgrav.c:403-428): C[k] = (centre, size).
@@ -626,34 +686,9 @@ __global__ void cells_kernel(const uint64_t* __restrict__ keys, int words, int64
   const int k = e.x;
   const int64_t i = e.y;
   const int L = lp[i] + 1 + (k - base[i]);
-  const int lsb_m = root->lsb_m, lsb_f = root->lsb_f;
-  const dvec4 C = na.C[k];
   const int64_t end = cell_end(keys, words, n, lp, i, L);
-  const int next = end < n ? base[end] : nnodes;
-  const double c[3] = {C.x, C.y, C.z};
-  float4 A, Lo;
-  A.x = f32_hi(c[0]);
-  A.y = f32_hi(c[1]);
-  A.z = f32_hi(c[2]);
-  A.w = (float)dmul(C.w, C.w);
-  Lo.x = f32_lo(c[0], A.x);
-  Lo.y = f32_lo(c[1], A.y);
-  Lo.z = f32_lo(c[2], A.z);
-  Lo.w = __int_as_float(next);
-  na.R[k].A = A;
-  na.R[k].L = Lo;
-  // monopole of particles [i, end): exact sums, one rounding each, then
-  // firstmoment / mass (_jbgrav.c:478) with a Newton-refined reciprocal
-  const FxMoments Pi = fxm_prefix(fx_local, fx_tiles, i, n);
-  const FxMoments Pe = fxm_prefix(fx_local, fx_tiles, end, n);
-  const double cm = fx::to_double(fx::sub(Pe.c[0], Pi.c[0]), lsb_m);
-  const double r = rcp_f64(cm);
-  double com[3];
-#pragma unroll
-  for (int a2 = 0; a2 < 3; a2++) com[a2] = dmul(fx::to_double(fx::sub(Pe.c[a2 + 1], Pi.c[a2 + 1]), lsb_f), r);
-  na.M[k] = make_dvec4(com[0], com[1], com[2], cm);
-  na.R[k].O = make_float4((float)dsub(com[0], c[0]), (float)dsub(com[1], c[1]), (float)dsub(com[2], c[2]),
-                          (float)cm);
+  write_cell(na, k, end < n ? base[end] : nnodes, na.C[k], i, end, n, root->lsb_m, root->lsb_f, fx_local, fx_tiles,
+             MS_BITS);
 }
 
 // ---------------------------------------------------------------------------
@@ -685,10 +720,11 @@ __device__ __forceinline__ FxMoments particle_moments(const double* __restrict__
   return r;
 }
 
-// Exclusive scan of the threads' totals within a block of MS_THREADS; returns the
-// thread's exclusive prefix.
+// Exclusive scan of the threads' totals within a block of T; returns the thread's
+// exclusive prefix.
+template <int T>
 __device__ __forceinline__ FxMoments fxm_block_exclusive(const FxMoments& tot) {
-  __shared__ FxMoments warp_tot[MS_THREADS / 32];
+  __shared__ FxMoments warp_tot[T / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   FxMoments inc = tot;
 #pragma unroll
@@ -710,22 +746,23 @@ __device__ __forceinline__ FxMoments fxm_block_exclusive(const FxMoments& tot) {
   return before;
 }
 
-// Per tile of MS_TILE key-ordered particles: the prefix of every particle within its
+// Per tile of MS_THREADS * ITEMS key-ordered particles: the prefix of every particle within its
 // tile (fx_local) and the tile's total (fx_tiles[tile]).
+template <int ITEMS>
 __global__ void __launch_bounds__(MS_THREADS)
     moments_scan_kernel(const double* __restrict__ pos, const double* __restrict__ mass,
                         const uint32_t* __restrict__ perm, int64_t n, const TreeRoot* __restrict__ root,
                         FxMoments* __restrict__ fx_local, FxMoments* __restrict__ fx_tiles) {
   const int lsb_m = root->lsb_m, lsb_f = root->lsb_f;
-  const int64_t j0 = (int64_t)blockIdx.x * MS_TILE + (int64_t)threadIdx.x * MS_ITEMS;
+  const int64_t j0 = ((int64_t)blockIdx.x * MS_THREADS + threadIdx.x) * ITEMS;
   // each item's moments are formed twice (for the thread's total, then for the running
   // prefix): measured cheaper than storing them and reading them back (1.22 against
   // 1.33 ms per build at N = 1M)
   FxMoments tot = fxm_zero();
-  for (int r = 0; r < MS_ITEMS; r++)
+  for (int r = 0; r < ITEMS; r++)
     if (j0 + r < n) fxm_add(tot, particle_moments(pos, mass, perm[j0 + r], lsb_m, lsb_f));
-  FxMoments run = fxm_block_exclusive(tot);
-  for (int r = 0; r < MS_ITEMS; r++)
+  FxMoments run = fxm_block_exclusive<MS_THREADS>(tot);
+  for (int r = 0; r < ITEMS; r++)
     if (j0 + r < n) {
       fx_local[j0 + r] = run;
       fxm_add(run, particle_moments(pos, mass, perm[j0 + r], lsb_m, lsb_f));
@@ -740,13 +777,195 @@ __global__ void __launch_bounds__(MS_THREADS) moments_tiles_kernel(FxMoments* __
   const int64_t b = a + per < ntiles ? a + per : ntiles;
   FxMoments tot = fxm_zero();
   for (int64_t t = a; t < b; t++) fxm_add(tot, fx_tiles[t]);
-  FxMoments run = fxm_block_exclusive(tot);
+  FxMoments run = fxm_block_exclusive<MS_THREADS>(tot);
   for (int64_t t = a; t < b; t++) {
     const FxMoments v = fx_tiles[t];
     fx_tiles[t] = run;
     fxm_add(run, v);
   }
   if (threadIdx.x == MS_THREADS - 1) fx_tiles[ntiles] = run;
+}
+
+// ---------------------------------------------------------------------------
+// Build of a small system (n <= SB_MAX): a build of a few thousand particles is bound by
+// its 27 launches and by latency (250 us at N = 2000, whatever N down to 100), so here it
+// is six: box and root, keys, rank, moments, layout (one block) and cells.  The keys are sorted by
+// counting smaller ones, n^2 comparisons over all SMs.  Only the two-word keys are
+// handled: a tie, a non-finite input or more nodes than the caller's room leaves a status
+// and a tree of zero nodes, which the walk takes no step on.  The host reads the status
+// after the walk is queued, so the GPU does not wait for it.
+// ---------------------------------------------------------------------------
+constexpr int SB_MAX = 8192;
+constexpr int SB_ITEMS = SB_MAX / SB_THREADS;
+enum SmallStatus { SB_OK = 0, SB_BAD = 1, SB_TIE = 2, SB_ROOM = 3 };
+
+// Rank of each key among all (words and index), 16 particles x 16 slices of the others per
+// block; writes the keys and indices in order.
+constexpr int RK_THREADS = 256, RK_CHUNK = 1024;
+__global__ void __launch_bounds__(RK_THREADS)
+    small_rank_kernel(const uint64_t* __restrict__ kin, int n, uint64_t* __restrict__ kout, uint32_t* __restrict__ idx) {
+  __shared__ uint64_t c0[RK_CHUNK], c1[RK_CHUNK];
+  const int slice = threadIdx.x & 15, i = blockIdx.x * 16 + (threadIdx.x >> 4);
+  const uint64_t k0 = i < n ? kin[i] : 0ull, k1 = i < n ? kin[n + i] : 0ull;
+  int rank = 0;
+  for (int b = 0; b < n; b += RK_CHUNK) {
+    const int m = n - b < RK_CHUNK ? n - b : RK_CHUNK;
+    __syncthreads();
+    for (int q = threadIdx.x; q < m; q += RK_THREADS) {
+      c0[q] = kin[b + q];
+      c1[q] = kin[n + b + q];
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int q = slice; q < m; q += 16) {
+      const uint64_t a0 = c0[q], a1 = c1[q];
+      rank += a0 < k0 || (a0 == k0 && (a1 < k1 || (a1 == k1 && b + q < i)));
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+  if (slice == 0 && i < n) {
+    kout[rank] = k0;
+    kout[n + rank] = k1;
+    idx[rank] = (uint32_t)i;
+  }
+}
+
+// Common prefixes, the nodes' places in the preorder (base; base[n] = nodes, or 0 with a
+// status) and the prefixes of the moment tiles, in one block; thread t has the contiguous
+// key-ordered particles from t * per on.
+__global__ void __launch_bounds__(SB_THREADS)
+    small_layout_kernel(const uint64_t* __restrict__ keys, int n, int room, const TreeRoot* __restrict__ root,
+                        int* __restrict__ lp, int* __restrict__ base, FxMoments* __restrict__ fx_tiles,
+                        int* __restrict__ status) {
+  __shared__ int warp_sum[SB_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (n + SB_THREADS - 1) / SB_THREADS;
+  const int j0 = tid * per < n ? tid * per : n, j1 = j0 + per < n ? j0 + per : n;
+  int l[SB_ITEMS + 1], cnt[SB_ITEMS];
+  bool tie = false;
+#pragma unroll
+  for (int r = 0; r <= SB_ITEMS; r++) {
+    const int j = j0 + r;
+    l[r] = -1;
+    if (r <= j1 - j0 && j > 0 && j < n) l[r] = key_lcp(keys, 2, n, j - 1, j);
+    tie = tie || l[r] >= 2 * KEY_LEVELS;
+  }
+  int mine = 0;
+#pragma unroll
+  for (int r = 0; r < SB_ITEMS; r++) {
+    cnt[r] = 1 + (l[r] > l[r + 1] ? l[r] : l[r + 1]) - l[r];
+    if (r < j1 - j0) mine += cnt[r];
+  }
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  tie = __syncthreads_or(tie);
+  int before = incl - mine, total = 0;
+  for (int w = 0; w < SB_THREADS / 32; w++) {
+    const int s = warp_sum[w];
+    if (w < warp) before += s;
+    total += s;
+  }
+#pragma unroll
+  for (int r = 0; r < SB_ITEMS; r++)
+    if (r < j1 - j0) {
+      lp[j0 + r] = l[r];
+      base[j0 + r] = before;
+      before += cnt[r];
+    }
+  if (tid == 0) {
+    const int st = root->bad ? SB_BAD : (tie ? SB_TIE : (total > room ? SB_ROOM : SB_OK));
+    lp[n] = -1;
+    base[n] = st == SB_OK ? total : 0;
+    status[1] = total;
+    status[0] = st;
+  }
+  if (warp == 1) {  // tile totals -> prefixes: at most 32 tiles
+    static_assert(SB_MAX >> SB_BITS <= 32, "one warp scans the tiles");
+    const int ntiles = ((n - 1) >> SB_BITS) + 1;
+    const FxMoments v = lane < ntiles ? fx_tiles[lane] : fxm_zero();
+    FxMoments inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      FxMoments y;
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int w = 0; w < 3; w++) y.c[k].w[w] = __shfl_up_sync(0xffffffffu, inc.c[k].w[w], d);
+      if (lane >= d) fxm_add(inc, y);
+    }
+    if (lane == ntiles - 1) fx_tiles[ntiles] = inc;
+#pragma unroll
+    for (int k = 0; k < 4; k++) inc.c[k] = fx::sub(inc.c[k], v.c[k]);
+    if (lane < ntiles) fx_tiles[lane] = inc;
+  }
+}
+
+// A block of key-ordered particles: their leaves and the centres of the internal cells
+// that they open, by the reference's FP64 recurrence along their digits (see nodes_kernel,
+// cell_centres_kernel), then the rest of those cells, one thread each: the block's nodes
+// are contiguous in the preorder.
+constexpr int SC_CELL_THREADS = 64;
+__global__ void __launch_bounds__(SC_CELL_THREADS)
+    small_cells_kernel(const double* __restrict__ pos, const double* __restrict__ mass,
+                       const uint64_t* __restrict__ keys, const uint32_t* __restrict__ perm, int n,
+                       const TreeRoot* __restrict__ root, const int* __restrict__ lp, const int* __restrict__ base,
+                       NodeArrays na, const FxMoments* __restrict__ fx_local, const FxMoments* __restrict__ fx_tiles) {
+  __shared__ double offs[2 * KEY_LEVELS], sizes[2 * KEY_LEVELS];
+  __shared__ int s_lp[SC_CELL_THREADS], s_base[SC_CELL_THREADS + 1];
+  const int tid = threadIdx.x, i0 = blockIdx.x * SC_CELL_THREADS, i = i0 + tid;
+  const int nnodes = base[n];
+  if (nnodes == 0) return;
+  const int m = n - i0 < SC_CELL_THREADS ? n - i0 : SC_CELL_THREADS;
+  if (tid < 2 * KEY_LEVELS) {
+    sizes[tid] = dmul(root->size, __longlong_as_double((long long)(1023 - tid) << 52));
+    offs[tid] = dmul(root->size, __longlong_as_double((long long)(1023 - (tid + 2)) << 52));
+  }
+  if (tid == 0) s_base[m] = base[i0 + m];
+  if (tid < m) {
+    s_lp[tid] = lp[i];
+    s_base[tid] = base[i];
+  }
+  __syncthreads();
+  if (tid < m) {
+    const int lo = s_lp[tid] + 1, k0 = s_base[tid], d = lo + s_base[tid + 1] - k0 - 1;
+    const int64_t p = perm[i];
+    write_leaf(na, k0 + (d - lo), k0 + (d - lo) + 1, pos[3 * p], pos[3 * p + 1], pos[3 * p + 2], mass[p]);
+    if (d > lo) {
+      const uint64_t kw0 = keys[i], kw1 = keys[n + i];
+      double c[3] = {root->c[0], root->c[1], root->c[2]};
+      for (int L = 0; L < d; L++) {
+        if (L >= lo) na.C[k0 + (L - lo)] = make_dvec4(c[0], c[1], c[2], sizes[L]);
+        if (L + 1 < d) {
+          const unsigned g = L < KEY_LEVELS ? (unsigned)(kw0 >> (3 * (KEY_LEVELS - 1 - L))) & 7u
+                                            : (unsigned)(kw1 >> (3 * (2 * KEY_LEVELS - 1 - L))) & 7u;
+          const double off = offs[L];
+#pragma unroll
+          for (int r = 0; r < 3; r++) c[r] = dadd(c[r], ((g >> r) & 1u) ? off : -off);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const int lsb_m = root->lsb_m, lsb_f = root->lsb_f;
+  for (int k = s_base[0] + tid; k < s_base[m]; k += SC_CELL_THREADS) {
+    int a = 0, b = m - 1;  // the particle that opens node k: the last with base <= k
+    while (a < b) {
+      const int mid = (a + b + 1) >> 1;
+      if (s_base[mid] <= k)
+        a = mid;
+      else
+        b = mid - 1;
+    }
+    if (k == s_base[a + 1] - 1) continue;  // its leaf
+    const int64_t end = cell_end(keys, 2, n, lp, i0 + a, s_lp[a] + 1 + k - s_base[a]);
+    write_cell(na, k, end < n ? base[end] : nnodes, na.C[k], i0 + a, end, n, lsb_m, lsb_f, fx_local, fx_tiles, SB_BITS);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -888,10 +1107,12 @@ __device__ __forceinline__ bool walk_is_chain(const WalkRec* __restrict__ nR, in
 
 template <bool GUARD, bool STATS, class Epi>
 __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
-    tree_walk_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, int nnodes,
+    tree_walk_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, const int* __restrict__ nodes,
                      const double* __restrict__ tpos, const uint32_t* __restrict__ order, int64_t nt,
                      double eps2, double theta, float th2_lo, float th2_hi, Epi epi,
                      unsigned long long* __restrict__ stats) {
+  const int nnodes = *nodes;
+  if (nnodes == 0) return;  // a build that did not succeed
   const int64_t slot = (int64_t)blockIdx.x * TW_THREADS + threadIdx.x;
   const bool valid = slot < nt;
   const int64_t t = valid ? (order ? (int64_t)order[slot] : slot) : 0;
@@ -1023,9 +1244,11 @@ __device__ __forceinline__ int walk_bound(int s, int K, int own, int nnodes) {
 template <bool GUARD, bool STATS, bool SPLIT, class Epi>
 __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     tree_walk_f64_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, const dvec4* __restrict__ nM,
-                         int nnodes, const double* __restrict__ tpos, const uint32_t* __restrict__ order, int64_t nt,
-                         double eps2, double theta, float th2_lo, float th2_hi, Epi epi, WalkSplit sp,
-                         unsigned long long* __restrict__ stats) {
+                         const int* __restrict__ nodes, const double* __restrict__ tpos,
+                         const uint32_t* __restrict__ order, int64_t nt, double eps2, double theta, float th2_lo,
+                         float th2_hi, Epi epi, WalkSplit sp, unsigned long long* __restrict__ stats) {
+  const int nnodes = *nodes;
+  if (nnodes == 0) return;  // a build that did not succeed
   const int lane = threadIdx.x & 31;
   const unsigned set = SPLIT ? blockIdx.x / sp.segs : blockIdx.x;  // of neighbouring target groups
   const int seg = SPLIT ? (int)(blockIdx.x - set * sp.segs) : 0;
@@ -1166,7 +1389,10 @@ struct TreeWS {
   Buffer tkeys, tkeys_tmp, tidx, tidx_tmp, trs;  // target points' walk order
   Buffer list;                // particle lists: key fallbacks, then cell openers
   Buffer cells;               // (internal cell, opener) pairs
-  int* host_flags = nullptr;  // pinned: the 8 device flags, nnodes, the root's non-finite flag
+  int* host_flags = nullptr;  // pinned: the 8 device flags, nnodes, the root's non-finite flag; [10..11] small build
+  cudaEvent_t small_built = nullptr;
+  int64_t small_tie_n = -1;   // particle count of the last small build whose two-word keys tied
+  int64_t small_room = 0;     // nodes that a small build may write
   int words = TREE_MIN_WORDS;
   int64_t full_sort_n = -1;  // particle count whose last build needed the full multi-word sort
 };
@@ -1183,8 +1409,10 @@ static NodeArrays node_arrays(TreeWS& ws) {
 
 struct BuiltTree {
   int64_t n = 0;  // particles
-  int nnodes = 0;
+  int nnodes = 0;              // (unknown while pending)
   int maxdepth = 0;
+  const int* nodes = nullptr;  // the same on the device; 0 when the build did not succeed
+  bool pending = false;        // a small build whose status has not been read
   const uint32_t* torder = nullptr;  // target points in key order (when sorted)
 };
 
@@ -1194,24 +1422,107 @@ constexpr int64_t TGT_SORT_MIN = 8192;
 
 constexpr int64_t KEYS_WIDE = 4 * 152 * 256;
 
+static int bad_input() {
+  return set_error(GH_ERR_ARG,
+                   "tree: particle positions and masses must be finite (the reference's octree insert "
+                   "does not terminate on NaN or infinite coordinates)");
+}
+
+// Queues the build of a small system; small_finish reads its status.
+static int small_build(TreeWS& ws, const double* pos, const double* mass, int64_t n, double eps, cudaStream_t st,
+                       BuiltTree* out) {
+  if (!ws.small_built) GH_CUDA_TRY(cudaEventCreateWithFlags(&ws.small_built, cudaEventDisableTiming));
+  if (ws.small_room < 4 * n + 1024) ws.small_room = 4 * n + 1024;
+  const size_t room = (size_t)ws.small_room;
+  GH_TRY(ensure(ws.root, sizeof(TreeRoot)));
+  GH_TRY(ensure(ws.lp, (n + 1) * sizeof(int)));
+  GH_TRY(ensure(ws.base, (n + 1) * sizeof(int)));
+  GH_TRY(ensure(ws.idx, n * sizeof(uint32_t)));
+  GH_TRY(ensure(ws.idx_tmp, n * sizeof(uint32_t)));
+  GH_TRY(ensure(ws.keys, (size_t)2 * n * sizeof(uint64_t)));
+  GH_TRY(ensure(ws.keys_tmp, (size_t)2 * n * sizeof(uint64_t)));
+  GH_TRY(ensure(ws.nA, room * sizeof(WalkRec)));
+  GH_TRY(ensure(ws.nC, room * sizeof(dvec4)));
+  GH_TRY(ensure(ws.nM, room * sizeof(dvec4)));
+  GH_TRY(ensure(ws.fxl, (size_t)n * sizeof(FxMoments)));
+  GH_TRY(ensure(ws.fxt, (size_t)(((n - 1) >> SB_BITS) + 2) * sizeof(FxMoments)));
+  TreeRoot* root = (TreeRoot*)ws.root.ptr;
+  uint64_t *keys = (uint64_t*)ws.keys.ptr, *ktmp = (uint64_t*)ws.keys_tmp.ptr;
+  uint32_t* idx = (uint32_t*)ws.idx.ptr;
+  int *lp = (int*)ws.lp.ptr, *base = (int*)ws.base.ptr;
+  FxMoments *fxl = (FxMoments*)ws.fxl.ptr, *fxt = (FxMoments*)ws.fxt.ptr;
+  box_root_kernel<<<1, SB_THREADS, 0, st>>>(pos, mass, n, eps, root);
+  GH_LAUNCH_CHECK();
+  keys_kernel<256><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(pos, n, root, 2, ktmp, (uint32_t*)ws.idx_tmp.ptr);
+  GH_LAUNCH_CHECK();
+  small_rank_kernel<<<(unsigned)((n + 15) / 16), RK_THREADS, 0, st>>>(ktmp, (int)n, keys, idx);
+  GH_LAUNCH_CHECK();
+  moments_scan_kernel<1><<<(unsigned)((n + MS_THREADS - 1) / MS_THREADS), MS_THREADS, 0, st>>>(pos, mass, idx, n, root,
+                                                                                               fxl, fxt);
+  GH_LAUNCH_CHECK();
+  small_layout_kernel<<<1, SB_THREADS, 0, st>>>(keys, (int)n, (int)ws.small_room, root, lp, base, fxt,
+                                                ws.host_flags + 10);
+  GH_LAUNCH_CHECK();
+  GH_CUDA_TRY(cudaEventRecord(ws.small_built, st));
+  small_cells_kernel<<<(unsigned)((n + SC_CELL_THREADS - 1) / SC_CELL_THREADS), SC_CELL_THREADS, 0, st>>>(
+      pos, mass, keys, idx, (int)n, root, lp, base, node_arrays(ws), fxl, fxt);
+  GH_LAUNCH_CHECK();
+  out->n = n;
+  out->nodes = base + n;
+  out->pending = true;
+  return GH_OK;
+}
+
+// Waits for a small build's status.  *again: it did not succeed for a reason that the next
+// tree_build of the same particles takes care of (a walk queued on it has done nothing).
+static int small_finish(TreeWS& ws, BuiltTree* bt, bool* again) {
+  *again = false;
+  if (!bt->pending) return GH_OK;
+  bt->pending = false;
+  GH_CUDA_TRY(cudaEventSynchronize(ws.small_built));
+  const volatile int* status = ws.host_flags + 10;
+  bt->nnodes = status[1];
+  switch (status[0]) {
+    case SB_OK: return GH_OK;
+    case SB_BAD: return bad_input();
+    case SB_TIE: ws.small_tie_n = bt->n; break;
+    default: ws.small_room = (int64_t)status[1] + status[1] / 4;
+  }
+  *again = true;
+  return GH_OK;
+}
+
+
+// `defer`: a small system's build may be left pending (small_finish after the walk).
 static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t n, double eps,
-                      cudaStream_t st, BuiltTree* out, const double* tpos = nullptr, int64_t nt = 0) {
+                      cudaStream_t st, BuiltTree* out, bool defer = false, const double* tpos = nullptr,
+                      int64_t nt = 0) {
   Trace tr("tree build");
+  *out = BuiltTree();
   const bool sort_targets = tpos != nullptr && nt >= TGT_SORT_MIN;
   if (sort_targets && nt > (1LL << 31))
     return set_error(GH_ERR_ARG, "tree: at most 2^31 target points (got %lld)", (long long)nt);
   // int32 node indices: at most 127 cells per particle
   if (n > (1LL << 24)) return set_error(GH_ERR_ARG, "tree: at most 16777216 particles (got %lld)", (long long)n);
   if (!ws.host_flags) GH_CUDA_TRY(cudaMallocHost((void**)&ws.host_flags, 16 * sizeof(int)));
+  const bool wait_fault = inject_take(GH_INJECT_TREE_WAIT);  // test hook: as if a look-back wait had run out
+  if (n <= SB_MAX && n != ws.small_tie_n && !sort_targets && !wait_fault) {
+    GH_TRY(small_build(ws, pos, mass, n, eps, st, out));
+    if (defer) return GH_OK;
+    bool again;
+    GH_TRY(small_finish(ws, out, &again));
+    if (!again) return GH_OK;
+    return tree_build(ws, pos, mass, n, eps, st, out, false, tpos, nt);
+  }
   const int T = 256;
   // 1. root cell
-  GH_TRY(ensure(ws.part, BB_BLOCKS * BB_PART * sizeof(double)));
+  GH_TRY(ensure(ws.part, BB_BLOCKS * sizeof(Box)));
   GH_TRY(ensure(ws.root, sizeof(TreeRoot)));
   int nb = (int)((n + BB_THREADS - 1) / BB_THREADS);
   if (nb > BB_BLOCKS) nb = BB_BLOCKS;
-  bbox_partial_kernel<<<nb, BB_THREADS, 0, st>>>(pos, mass, n, (double*)ws.part.ptr);
+  bbox_partial_kernel<<<nb, BB_THREADS, 0, st>>>(pos, mass, n, (Box*)ws.part.ptr);
   GH_LAUNCH_CHECK();
-  root_kernel<<<1, 32, 0, st>>>((const double*)ws.part.ptr, nb, eps, (TreeRoot*)ws.root.ptr);
+  root_kernel<<<1, 32, 0, st>>>((const Box*)ws.part.ptr, nb, eps, (TreeRoot*)ws.root.ptr);
   GH_LAUNCH_CHECK();
   const TreeRoot* root = (const TreeRoot*)ws.root.ptr;
   const unsigned gn = (unsigned)((n + T - 1) / T), gn1 = (unsigned)((n + 1 + T - 1) / T);
@@ -1259,7 +1570,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
       tie_copy_kernel<<<gn, T, 0, st>>>(keys, words, n, idx, ktmp, itmp);
       GH_LAUNCH_CHECK();
     }
-    if (inject_take(GH_INJECT_TREE_WAIT))  // test hook: as if a look-back wait had run out
+    if (wait_fault)
       GH_CUDA_TRY(cudaMemsetAsync(flags + 5, 1, 1, st));
     lcp_kernel<<<gn1, T, 0, st>>>(keys, words, n, (int*)ws.lp.ptr, (int*)ws.flags.ptr);
     GH_LAUNCH_CHECK();
@@ -1287,10 +1598,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
     GH_CUDA_TRY(cudaStreamSynchronize(st));
     // The kernels so far index only by particle and sort slot, whatever the keys hold,
     // so non-finite input is refused here, before any cell is built from it.
-    if (ws.host_flags[9])
-      return set_error(GH_ERR_ARG,
-                       "tree: particle positions and masses must be finite (the reference's octree insert "
-                       "does not terminate on NaN or infinite coordinates)");
+    if (ws.host_flags[9]) return bad_input();
     if (ws.host_flags[5]) return set_error(GH_ERR_TIMEOUT, "tree: radix sort look-back gave up");
     if (ws.host_flags[2] && !full_sort) {  // a long run of equal first words
       full_sort = true;
@@ -1328,7 +1636,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
     FxMoments* fxl = (FxMoments*)ws.fxl.ptr;
     FxMoments* fxt = (FxMoments*)ws.fxt.ptr;
     // 5. exact prefix sums of the moments (the cells' monopoles come from them below)
-    moments_scan_kernel<<<(unsigned)ntiles, MS_THREADS, 0, st>>>(pos, mass, perm, n, root, fxl, fxt);
+    moments_scan_kernel<MS_ITEMS><<<(unsigned)ntiles, MS_THREADS, 0, st>>>(pos, mass, perm, n, root, fxl, fxt);
     GH_LAUNCH_CHECK();
     moments_tiles_kernel<<<1, MS_THREADS, 0, st>>>(fxt, ntiles);
     GH_LAUNCH_CHECK();
@@ -1348,6 +1656,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
   }
   out->n = n;
   out->nnodes = nnodes;
+  out->nodes = (const int*)ws.base.ptr + n;
   out->maxdepth = maxdepth;
   return GH_OK;
 }
@@ -1415,14 +1724,14 @@ static int launch_walk_f64(TreeWS& ws, const NodeArrays& na, const BuiltTree& bt
   }
   prof_begin(st);
   if (stats)
-    tree_walk_f64_kernel<G, true, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nnodes, tpos, order,
+    tree_walk_f64_kernel<G, true, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nodes, tpos, order,
                                                                              nt, eps2, theta, lo, hi, epi, sp, stats);
   else if (sp.segs > 1)
-    tree_walk_f64_kernel<G, false, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nnodes, tpos, order,
+    tree_walk_f64_kernel<G, false, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, na.M, bt.nodes, tpos, order,
                                                                              nt, eps2, theta, lo, hi, epi, sp, nullptr);
   else
     tree_walk_f64_kernel<G, false, false, Epi><<<blocks, TW_THREADS, 0, st>>>(
-        na.R, na.C, na.M, bt.nnodes, tpos, order, nt, eps2, theta, lo, hi, epi, sp, nullptr);
+        na.R, na.C, na.M, bt.nodes, tpos, order, nt, eps2, theta, lo, hi, epi, sp, nullptr);
   prof_end(st);
   return GH_OK;
 }
@@ -1434,10 +1743,10 @@ static void launch_walk_mixed(const NodeArrays& na, const BuiltTree& bt, const d
   const unsigned blocks = (unsigned)((nt + TW_THREADS - 1) / TW_THREADS);
   prof_begin(st);
   if (stats)
-    tree_walk_kernel<G, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, bt.nnodes, tpos, order, nt, eps2, theta,
+    tree_walk_kernel<G, true, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, bt.nodes, tpos, order, nt, eps2, theta,
                                                                   lo, hi, epi, stats);
   else
-    tree_walk_kernel<G, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, bt.nnodes, tpos, order, nt, eps2, theta,
+    tree_walk_kernel<G, false, Epi><<<blocks, TW_THREADS, 0, st>>>(na.R, na.C, bt.nodes, tpos, order, nt, eps2, theta,
                                                                    lo, hi, epi, nullptr);
   prof_end(st);
 }
@@ -1509,11 +1818,17 @@ int tree_force(const double* pos, const double* mass, int64_t np, const double* 
   DeviceInfo di;
   GH_TRY(device_info(&di));
   TreeWS& ws = g_tree[di.device];
-  BuiltTree bt;
-  GH_TRY(tree_build(ws, pos, mass, np, eps, st, &bt, self ? nullptr : tpos, self ? 0 : nt));
   EpiStore epi{acc};
-  if (self) return tree_walk(ws, bt, pos, (const uint32_t*)ws.idx.ptr, np, true, eps, theta, precision, epi, st);
-  return tree_walk(ws, bt, tpos, bt.torder, nt, false, eps, theta, precision, epi, st);
+  for (bool again = true; again;) {
+    BuiltTree bt;
+    GH_TRY(tree_build(ws, pos, mass, np, eps, st, &bt, !g_stats_on, self ? nullptr : tpos, self ? 0 : nt));
+    if (self)
+      GH_TRY(tree_walk(ws, bt, pos, (const uint32_t*)ws.idx.ptr, np, true, eps, theta, precision, epi, st));
+    else
+      GH_TRY(tree_walk(ws, bt, tpos, bt.torder, nt, false, eps, theta, precision, epi, st));
+    GH_TRY(small_finish(ws, &bt, &again));
+  }
+  return GH_OK;
 }
 
 int tree_run(double* x, double* v, const double* mass, int64_t np, int64_t nsteps, double dt, double eps,
@@ -1530,8 +1845,6 @@ int tree_run(double* x, double* v, const double* mass, int64_t np, int64_t nstep
     Trace step("tree dkd step");
     const int cur = (int)(s & 1), nxt = cur ^ 1;
     const double* xh = (const double*)ws.xh[cur].ptr;
-    BuiltTree bt;
-    GH_TRY(tree_build(ws, xh, mass, np, eps, st, &bt));
     EpiDKD epi;
     epi.x = x;
     epi.v = v;
@@ -1546,7 +1859,12 @@ int tree_run(double* x, double* v, const double* mass, int64_t np, int64_t nstep
       epi.hist_x = hist_x + slot * np * 3;
       epi.hist_v = hist_v + slot * np * 3;
     }
-    GH_TRY(tree_walk(ws, bt, xh, (const uint32_t*)ws.idx.ptr, np, true, eps, theta, precision, epi, st));
+    for (bool again = true; again;) {
+      BuiltTree bt;
+      GH_TRY(tree_build(ws, xh, mass, np, eps, st, &bt, !g_stats_on));
+      GH_TRY(tree_walk(ws, bt, xh, (const uint32_t*)ws.idx.ptr, np, true, eps, theta, precision, epi, st));
+      GH_TRY(small_finish(ws, &bt, &again));
+    }
   }
   return GH_OK;
 }
