@@ -577,26 +577,45 @@ __global__ void __launch_bounds__(THREADS, MINB)
     __syncthreads();
     if (!s_last) continue;
     __threadfence();
+    // The partials of CTAs g_first .. g_last in that order, RG of this thread's targets at
+    // a time (one target at a time, with the two 64-bit divisions of each CTA's range
+    // start in its loop, took 45 of a step's 180 us at N = 16,384).  A CTA's first tile is
+    // in its slot 0: this tile is the first of every CTA but possibly g_first, whose range
+    // may begin in an earlier tile.
+    constexpr int RG = R > 4 ? R / 2 : R;
+    const int64_t first_slot = 2 * g_first + (t == sk_start(sk, g_first) / sk.chunks ? 0 : 1);
+    const int parts = (int)(g_last - g_first) + 1;
+    for (int r0 = 0; r0 < R; r0 += RG) {
+      float h[RG][3], l[RG][3];
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int64_t i = t * TILE + r * THREADS + tid;
-      float h[3] = {0.f, 0.f, 0.f}, l[3] = {0.f, 0.f, 0.f};
-      for (int64_t gg = g_first; gg <= g_last; gg++) {
-        const int64_t ft = sk_start(sk, gg) / sk.chunks;
-        const float* sl = partials + (2 * gg + (t == ft ? 0 : 1)) * SLOT;
+      for (int r = 0; r < RG; r++)
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-          float ph = __ldcg(sl + (int64_t)(2 * k) * TILE + r * THREADS + tid);
-          float pl = __ldcg(sl + (int64_t)(2 * k + 1) * TILE + r * THREADS + tid);
-          float s, e;
-          two_sum(h[k], ph, s, e);
-          h[k] = s;
-          l[k] = __fadd_rn(l[k], __fadd_rn(pl, e));
-        }
+        for (int k = 0; k < 3; k++) h[r][k] = l[r][k] = 0.f;
+      const float* sl = partials + first_slot * SLOT + r0 * THREADS + tid;
+      const float* rest = partials + 2 * (g_first + 1) * SLOT + r0 * THREADS + tid;
+#pragma unroll 2
+      for (int q = 0; q < parts; q++) {
+#pragma unroll
+        for (int r = 0; r < RG; r++)
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            const float ph = __ldcg(sl + (2 * k) * TILE + r * THREADS);
+            const float pl = __ldcg(sl + (2 * k + 1) * TILE + r * THREADS);
+            float s, e;
+            two_sum(h[r][k], ph, s, e);
+            h[r][k] = s;
+            l[r][k] = __fadd_rn(l[r][k], __fadd_rn(pl, e));
+          }
+        sl = rest;
+        rest += 2 * SLOT;
       }
-      if (i < nt)
-        epi(i, msc * ((double)h[0] + (double)l[0]), msc * ((double)h[1] + (double)l[1]),
-            msc * ((double)h[2] + (double)l[2]));
+#pragma unroll
+      for (int r = 0; r < RG; r++) {
+        const int64_t i = t * TILE + (r0 + r) * THREADS + tid;
+        if (i < nt)
+          epi(i, msc * ((double)h[r][0] + (double)l[r][0]), msc * ((double)h[r][1] + (double)l[r][1]),
+              msc * ((double)h[r][2] + (double)l[r][2]));
+      }
     }
     if (tid == 0) counters[t] = 0;  // ready for the next launch
   }
