@@ -116,8 +116,12 @@ static std::recursive_mutex g_mu;
 static int g_mixed_shape = -1;
 static int g_f64_form = -1;  // -1 by target count, 0 thread per target, 1 ordered CTA-wide terms
 
-// Chosen from a sweep of the shapes on GB300 (force and fused leapfrog step, N = 2048
-// to 1M): small systems want small tiles (more CTAs share the sources); from N ~ 24k
+// Chosen from a sweep of the shapes on GB300 (force and fused leapfrog step, N = 500 to
+// 1M): small systems want small tiles (more CTAs share the sources, and the FP64 epilogue
+// of a tile runs on more SMs: 8.5 us for 512 targets on one).  64 threads x 2 targets with
+// chunks of 256 (128 from N = 12,288): a step of N = 1000 takes 19 us against 28 with 256
+// x 2, 8192 52 against 65, 12,000 83 against 99; 16,384 132 against 140 with 128 x 4,
+// 20,000 188 against 206.  From N ~ 24k
 // the scalar FP32 loop with wide CTAs wins, 512 threads x 4 targets for a force at
 // every size (e.g. 1.78 ms against 1.93 ms for the packed 128 x 4 at N = 65,536) and
 // for the leapfrog step up to ~128k, 384 threads x 6 targets for larger steps, whose
@@ -152,25 +156,25 @@ static int auto_shape(int64_t np, int64_t nt, bool dkd) {
   const int64_t n = np > nt ? np : nt;
   const int tuned = tuned_shape(n, dkd);
   if (tuned >= 0) return tuned;
-  if (n < 12288) return 7;                   // packed, 256 threads, 1 pack, 4 CTAs/SM
-  if (n < 24576) return 3;                   // packed, 128 threads, 2 packs, 4 CTAs/SM
+  if (n < 12288) return 13;                  // packed, 64 threads, 1 pack, 8 CTAs/SM, chunks of 256
+  if (n < 24576) return 14;                  // the same, chunks of 128
   if (dkd && n >= (1 << 17)) return 12;      // scalar, 384 threads x 6 targets
   return 10;                                 // scalar, 512 threads x 4 targets
 }
 
-template <bool G, int T, int P, int B, class Epi, bool PK = true>
+template <bool G, int T, int P, int B, class Epi, bool PK = true, int JT = T>
 static int launch_shape(const StreamK& sk, const float4* src, int64_t np, const float4* tgt, int64_t nt,
                         float eps2, float* partials, int* counters, const Epi& epi, const double* eqm,
                         cudaStream_t st) {
-  direct_mixed_kernel<G, T, P, B, Epi, PK><<<(unsigned)sk.grid, T, 0, st>>>(src, np, tgt, nt, eps2, sk, partials,
+  direct_mixed_kernel<G, T, P, B, Epi, PK, JT><<<(unsigned)sk.grid, T, 0, st>>>(src, np, tgt, nt, eps2, sk, partials,
                                                                             counters, epi, eqm);
   return GH_OK;
 }
 
-template <bool G, int T, int P, int B, bool PK = true>
+template <bool G, int T, int P, int B, bool PK = true, int JT = T>
 static int occupancy_shape() {
   int o = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, direct_mixed_kernel<G, T, P, B, EpiStore, PK>, T, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, direct_mixed_kernel<G, T, P, B, EpiStore, PK, JT>, T, 0) !=
           cudaSuccess ||
       o < 1)
     o = 1;
@@ -194,7 +198,9 @@ static int dispatch_shape(int shape, const StreamK& sk, const float4* src, int64
     case 9: return launch_shape<G, 256, 2, 2, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
     case 10: return launch_shape<G, 512, 2, 1, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
     case 11: return launch_shape<G, 256, 4, 1, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
-    default: return launch_shape<G, 384, 3, 1, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
+    case 12: return launch_shape<G, 384, 3, 1, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
+    case 13: return launch_shape<G, 64, 1, 8, Epi, true, 256>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
+    default: return launch_shape<G, 64, 1, 8, Epi, true, 128>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
   }
 }
 
@@ -219,9 +225,11 @@ static int mixed_grid_cap(int num_sms, int shape, bool guard) {
       case 11:
         o = guard ? occupancy_shape<true, 256, 4, 1, false>() : occupancy_shape<false, 256, 4, 1, false>();
         break;
-      default:
+      case 12:
         o = guard ? occupancy_shape<true, 384, 3, 1, false>() : occupancy_shape<false, 384, 3, 1, false>();
         break;
+      case 13: o = guard ? occupancy_shape<true, 64, 1, 8, true, 256>() : occupancy_shape<false, 64, 1, 8, true, 256>(); break;
+      default: o = guard ? occupancy_shape<true, 64, 1, 8, true, 128>() : occupancy_shape<false, 64, 1, 8, true, 128>(); break;
     }
   }
   return o * num_sms;
@@ -314,7 +322,7 @@ static int launch_mixed(DirectWS& ws, const float4* src, int64_t np, const float
   const int shape = g_mixed_shape >= 0 ? g_mixed_shape : auto_shape(np, nt, Epi::kFusedStep);
   const MixedShape ms = kMixedShapes[shape];
   StreamK sk = mixed_plan(np, nt, mixed_grid_cap(di.num_sms, shape, guard), ms.threads * 2 * ms.packs,
-                          ms.threads);
+                          ms.jt);
   if (sk.units == 0) return GH_OK;
   GH_TRY(ensure_streamk(ws, sk, mixed_slot_floats(ms.threads, ms.packs), st));
   float* partials = (float*)ws.partials.ptr;

@@ -298,15 +298,19 @@ __global__ void __launch_bounds__(F64O_THREADS)
 // the CTA that finishes last (per-tile counter) combines them in CTA order, so
 // the result does not depend on timing, and runs the epilogue.
 // ---------------------------------------------------------------------------
-// Tile shapes of the mixed kernel: THREADS per CTA (also the sources per
-// shared-memory chunk), P f32x2 packs (2P targets) per thread, MINB CTAs per SM.
+// Tile shapes of the mixed kernel: THREADS per CTA, P f32x2 packs (2P targets) per thread,
+// MINB CTAs per SM, JT sources per chunk (a multiple of THREADS).  A chunk is both what
+// shared memory holds and what is summed in plain FP32, so JT alone decides a result's
+// FP32 rounding: shapes of one JT agree to the two-sums' 2^-48.
 struct MixedShape {
-  int threads, packs, minb;
+  int threads, packs, minb, jt;
 };
-constexpr MixedShape kMixedShapes[] = {{256, 2, 2}, {256, 4, 1}, {128, 4, 2}, {128, 2, 4}, {512, 2, 1},
-                                       {256, 2, 3}, {128, 2, 6}, {256, 1, 4}, {512, 2, 2},
-                                       {256, 2, 2}, {512, 2, 1}, {256, 4, 1}, {384, 3, 1}};
-// Shapes 9-12 run the scalar FP32 loop (mixed_chunk_scalar); 0-8 the packed f32x2 loop.
+constexpr MixedShape kMixedShapes[] = {{256, 2, 2, 256}, {256, 4, 1, 256}, {128, 4, 2, 128}, {128, 2, 4, 128},
+                                       {512, 2, 1, 512}, {256, 2, 3, 256}, {128, 2, 6, 128}, {256, 1, 4, 256},
+                                       {512, 2, 2, 512}, {256, 2, 2, 256}, {512, 2, 1, 512}, {256, 4, 1, 256},
+                                       {384, 3, 1, 384}, {64, 1, 8, 256}, {64, 1, 8, 128}};
+// Shapes 9-12 run the scalar FP32 loop (mixed_chunk_scalar); the others the packed f32x2
+// loop.
 constexpr int kNumMixedShapes = (int)(sizeof(kMixedShapes) / sizeof(kMixedShapes[0]));
 
 struct StreamK {
@@ -435,12 +439,14 @@ __host__ __device__ constexpr int64_t mixed_slot_floats(int threads, int packs) 
   return (int64_t)6 * threads * 2 * packs;
 }
 
-template <bool GUARD, int THREADS, int P, int MINB, class Epi, bool PACKED = true>
+template <bool GUARD, int THREADS, int P, int MINB, class Epi, bool PACKED = true, int JT = THREADS>
 __global__ void __launch_bounds__(THREADS, MINB)
     direct_mixed_kernel(const float4* __restrict__ src, int64_t np, const float4* __restrict__ tgt,
                         int64_t nt, float eps2, StreamK sk, float* __restrict__ partials,
                         int* __restrict__ counters, Epi epi, const double* __restrict__ eqm) {
-  constexpr int R = 2 * P, TILE = THREADS * R, JT = THREADS;
+  constexpr int R = 2 * P, TILE = THREADS * R;
+  constexpr int JS = JT / THREADS;  // sources of a chunk staged by each thread
+  static_assert(JT % THREADS == 0, "whole rows of sources");
   constexpr int64_t SLOT = mixed_slot_floats(THREADS, P);
   // Sources duplicated per lane pair: (x,x,y,y) and (z,z,m,m).
   __shared__ __align__(16) float4 tile[2 * 2 * JT];
@@ -489,26 +495,30 @@ __global__ void __launch_bounds__(THREADS, MINB)
     // source) instead of its mass: the equal-mass loop, which ignores w, runs only on
     // full chunks, and the general loop on the partial last chunk then gives r^-3 d
     // for a source and exactly 0 for padding.
-    float4 pre;
-    {
-      const int64_t j = c0 * JT + tid;
-      pre = j < np ? src[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-      if (eq) pre.w = j < np ? 1.f : 0.f;
-    }
+    float4 pre[JS];
+    auto load = [&](int64_t c) {
+#pragma unroll
+      for (int q = 0; q < JS; q++) {
+        const int64_t j = c * JT + q * THREADS + tid;
+        pre[q] = j < np ? src[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (eq) pre[q].w = j < np ? 1.f : 0.f;
+      }
+    };
+    load(c0);
     for (int64_t c = c0; c < c1; c++) {
       float4* tb = tile + buf * (2 * JT);
-      if (PACKED) {
-        tb[2 * tid + 0] = make_float4(pre.x, pre.x, pre.y, pre.y);
-        tb[2 * tid + 1] = make_float4(pre.z, pre.z, pre.w, pre.w);
-      } else {
-        tb[tid] = pre;
+#pragma unroll
+      for (int q = 0; q < JS; q++) {
+        const int k = q * THREADS + tid;
+        if (PACKED) {
+          tb[2 * k + 0] = make_float4(pre[q].x, pre[q].x, pre[q].y, pre[q].y);
+          tb[2 * k + 1] = make_float4(pre[q].z, pre[q].z, pre[q].w, pre[q].w);
+        } else {
+          tb[k] = pre[q];
+        }
       }
       __syncthreads();
-      if (c + 1 < c1) {
-        const int64_t j = (c + 1) * JT + tid;
-        pre = j < np ? src[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (eq) pre.w = j < np ? 1.f : 0.f;
-      }
+      if (c + 1 < c1) load(c + 1);
       const bool eq_loop = eq && (c + 1) * JT <= np;  // a full chunk of equal masses
       if (PACKED) {
         if (eq_loop)
