@@ -121,11 +121,16 @@ static int g_f64_form = -1;  // -1 by target count, 0 thread per target, 1 order
 // of a tile runs on more SMs: 8.5 us for 512 targets on one).  64 threads x 2 targets with
 // chunks of 256 (128 from N = 12,288): a step of N = 1000 takes 19 us against 28 with 256
 // x 2, 8192 52 against 65, 12,000 83 against 99; 16,384 132 against 140 with 128 x 4,
-// 20,000 188 against 206.  From N ~ 24k
-// the scalar FP32 loop with wide CTAs wins, 512 threads x 4 targets for a force at
-// every size (e.g. 1.78 ms against 1.93 ms for the packed 128 x 4 at N = 65,536) and
-// for the leapfrog step up to ~128k, 384 threads x 6 targets for larger steps, whose
-// heavier epilogue favours it (435 ms per step at N = 1M against 443 ms).
+// 20,000 188 against 206.  From N ~ 24k the scalar FP32 loop with wide CTAs wins, 512
+// threads x 4 targets for a force at every size (e.g. 1.78 ms against 1.93 ms for the
+// packed 128 x 4 at N = 65,536) and for the leapfrog step up to ~128k, 384 threads x 6
+// targets for larger steps, whose heavier epilogue favours it (435 ms per step at N = 1M
+// against 443 ms).
+//
+// Few points against many sources, or many against few, leave tiles of 2048 empty or SMs
+// idle: 64 threads x 2 targets with the same chunks of 512 takes 98 us against 240 for 10
+// to 100 points and 100,000 sources, 230 against 277 for 3000 points, 58 against 100 for
+// 50,000 points and 1000 sources; with 5000 sources it is slower (118 against 105).
 //
 // An autotuner can replace that table (gh_direct_tune): per epilogue kind (force or
 // fused leapfrog step), rules "from n_min particles on, shape k"; the rule with the
@@ -159,6 +164,7 @@ static int auto_shape(int64_t np, int64_t nt, bool dkd) {
   if (n < 12288) return 13;                  // packed, 64 threads, 1 pack, 8 CTAs/SM, chunks of 256
   if (n < 24576) return 14;                  // the same, chunks of 128
   if (dkd && n >= (1 << 17)) return 12;      // scalar, 384 threads x 6 targets
+  if (nt <= 4096 || np <= 2048) return 15;   // packed, 64 threads, 1 pack, 6 CTAs/SM, chunks of 512
   return 10;                                 // scalar, 512 threads x 4 targets
 }
 
@@ -200,7 +206,8 @@ static int dispatch_shape(int shape, const StreamK& sk, const float4* src, int64
     case 11: return launch_shape<G, 256, 4, 1, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
     case 12: return launch_shape<G, 384, 3, 1, Epi, false>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
     case 13: return launch_shape<G, 64, 1, 8, Epi, true, 256>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
-    default: return launch_shape<G, 64, 1, 8, Epi, true, 128>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
+    case 14: return launch_shape<G, 64, 1, 8, Epi, true, 128>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
+    default: return launch_shape<G, 64, 1, 6, Epi, true, 512>(sk, src, np, tgt, nt, eps2, partials, counters, epi, eqm, st);
   }
 }
 
@@ -229,7 +236,8 @@ static int mixed_grid_cap(int num_sms, int shape, bool guard) {
         o = guard ? occupancy_shape<true, 384, 3, 1, false>() : occupancy_shape<false, 384, 3, 1, false>();
         break;
       case 13: o = guard ? occupancy_shape<true, 64, 1, 8, true, 256>() : occupancy_shape<false, 64, 1, 8, true, 256>(); break;
-      default: o = guard ? occupancy_shape<true, 64, 1, 8, true, 128>() : occupancy_shape<false, 64, 1, 8, true, 128>(); break;
+      case 14: o = guard ? occupancy_shape<true, 64, 1, 8, true, 128>() : occupancy_shape<false, 64, 1, 8, true, 128>(); break;
+      default: o = guard ? occupancy_shape<true, 64, 1, 6, true, 512>() : occupancy_shape<false, 64, 1, 6, true, 512>(); break;
     }
   }
   return o * num_sms;

@@ -308,7 +308,7 @@ struct MixedShape {
 constexpr MixedShape kMixedShapes[] = {{256, 2, 2, 256}, {256, 4, 1, 256}, {128, 4, 2, 128}, {128, 2, 4, 128},
                                        {512, 2, 1, 512}, {256, 2, 3, 256}, {128, 2, 6, 128}, {256, 1, 4, 256},
                                        {512, 2, 2, 512}, {256, 2, 2, 256}, {512, 2, 1, 512}, {256, 4, 1, 256},
-                                       {384, 3, 1, 384}, {64, 1, 8, 256}, {64, 1, 8, 128}};
+                                       {384, 3, 1, 384}, {64, 1, 8, 256}, {64, 1, 8, 128}, {64, 1, 6, 512}};
 // Shapes 9-12 run the scalar FP32 loop (mixed_chunk_scalar); the others the packed f32x2
 // loop.
 constexpr int kNumMixedShapes = (int)(sizeof(kMixedShapes) / sizeof(kMixedShapes[0]));
