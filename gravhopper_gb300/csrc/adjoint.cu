@@ -273,23 +273,28 @@ __global__ void vjp_reduce_f64_kernel(const double* __restrict__ part, int split
   if (gmass) gmass[k] = a[3];
 }
 
-__global__ void vjp_reduce_mixed_kernel(const float* __restrict__ part, int splits, int64_t n,
+// One thread per target and component: (hi, lo) pairs are 8 bytes of consecutive threads,
+// and the splits' sums are added in split order (one thread per target with 4-byte loads 32
+// bytes apart took 41 us at N = 16,384, 32 splits).
+__global__ void vjp_reduce_mixed_kernel(const float2* __restrict__ part, int splits, int64_t n,
                                         const double* __restrict__ meqp, double* __restrict__ gpos,
                                         double* __restrict__ gmass) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  double a[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int s = 0; s < splits; s++)
-    for (int q = 0; q < 4; q++) {
-      const float* o = part + ((int64_t)s * n + k) * 8;
-      a[q] += (double)o[2 * q] + (double)o[2 * q + 1];
-    }
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 4 * n) return;
+  double a = 0.0;
+#pragma unroll 8
+  for (int s = 0; s < splits; s++) {
+    const float2 o = part[(int64_t)s * n * 4 + i];
+    a += (double)o.x + (double)o.y;
+  }
+  const int64_t k = i >> 2;
+  const int q = (int)(i & 3);
+  if (q == 3) {
+    if (gmass) gmass[k] = a;
+    return;
+  }
   const double meq = *meqp;
-  const double sm = meq != 0.0 ? meq : 1.0;  // equal masses: the sums were taken with unit masses
-  gpos[3 * k] = sm * a[0];
-  gpos[3 * k + 1] = sm * a[1];
-  gpos[3 * k + 2] = sm * a[2];
-  if (gmass) gmass[k] = a[3];
+  gpos[3 * k + q] = (meq != 0.0 ? meq : 1.0) * a;  // equal masses: the sums were taken with unit masses
 }
 
 // ---------------------------------------------------------------------------
@@ -391,38 +396,57 @@ __global__ void potential_reduce_kernel(const double* __restrict__ part_i, const
   phi[k] = a;
 }
 
-// FP32 relative sources (x, y, z, m) and cotangents (lx, ly, lz, 0).
-__global__ void vjp_prepare_mixed_kernel(const double* __restrict__ pos, const double* __restrict__ mass,
-                                         const double* __restrict__ lam, int64_t n, const double* __restrict__ origin,
-                                         float4* __restrict__ src, float4* __restrict__ lsrc) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  src[i] = make_float4((float)(pos[3 * i] - origin[0]), (float)(pos[3 * i + 1] - origin[1]),
-                       (float)(pos[3 * i + 2] - origin[2]), (float)mass[i]);
-  lsrc[i] = make_float4((float)lam[3 * i], (float)lam[3 * i + 1], (float)lam[3 * i + 2], 0.f);
-}
+// Mass-weighted centre for the FP32 sources, in 256 chains (particles t, t + 256, ...) of
+// FP64 sums and a fixed tree over the chains, and whether every mass equals the first
+// (finite, nonzero; a NaN never does).  One warp of chains per block: a block of all 256
+// ran its FP64 sums on one SM, one dependent load after another (37 us at N = 16,384).
+constexpr int MO_CHAINS = 256;
 
-// origin[0..2]: the mass-weighted centre; origin[3]: the common mass when every mass
-// equals the first (finite, nonzero; a NaN never does), else 0.
-__global__ void mean_origin_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n,
-                                   double* __restrict__ origin) {
-  __shared__ dvec4 red[256];
+__global__ void __launch_bounds__(32)
+    origin_chains_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n,
+                         dvec4* __restrict__ chain, int* __restrict__ differ) {
   const double m0 = n > 0 ? mass[0] : 0.0;
   dvec4 a = make_dvec4(0.0, 0.0, 0.0, 0.0);
   bool ne = false;
-  for (int64_t i = threadIdx.x; i < n; i += 256) {
-    const double m = mass[i];
-    ne |= !(m == m0);
-    a.x += m * pos[3 * i];
-    a.y += m * pos[3 * i + 1];
-    a.z += m * pos[3 * i + 2];
-    a.w += m;
+  constexpr int U = 8;  // loads in flight
+  for (int64_t i = blockIdx.x * 32 + threadIdx.x; i < n; i += U * MO_CHAINS) {
+    double m[U], x[U], y[U], z[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t j = i + u * MO_CHAINS < n ? i + u * MO_CHAINS : i;
+      m[u] = mass[j];
+      x[u] = pos[3 * j];
+      y[u] = pos[3 * j + 1];
+      z[u] = pos[3 * j + 2];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      ne |= !(m[u] == m0);
+      if (i + u * MO_CHAINS < n) {
+        a.x += m[u] * x[u];
+        a.y += m[u] * y[u];
+        a.z += m[u] * z[u];
+        a.w += m[u];
+      }
+    }
   }
-  ne = __syncthreads_or(ne);
-  if (threadIdx.x == 0) origin[3] = (!ne && m0 != 0.0 && isfinite(m0)) ? m0 : 0.0;
-  red[threadIdx.x] = a;
+  chain[blockIdx.x * 32 + threadIdx.x] = a;
+  ne = __any_sync(0xffffffffu, ne);
+  if (threadIdx.x == 0) differ[blockIdx.x] = ne;
+}
+
+// FP32 relative sources (x, y, z, m) and cotangents (lx, ly, lz, 0).  Every block adds the
+// chains up for itself; block 0 leaves the centre in origin[0..2] and the common mass (0
+// when the masses differ) in origin[3].
+__global__ void __launch_bounds__(MO_CHAINS)
+    vjp_prepare_mixed_kernel(const double* __restrict__ pos, const double* __restrict__ mass,
+                             const double* __restrict__ lam, int64_t n, const dvec4* __restrict__ chain,
+                             const int* __restrict__ differ, double* __restrict__ origin, float4* __restrict__ src,
+                             float4* __restrict__ lsrc) {
+  __shared__ dvec4 red[MO_CHAINS];
+  red[threadIdx.x] = chain[threadIdx.x];
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
+  for (int s = MO_CHAINS / 2; s > 0; s >>= 1) {
     if (threadIdx.x < s) {
       red[threadIdx.x].x += red[threadIdx.x + s].x;
       red[threadIdx.x].y += red[threadIdx.x + s].y;
@@ -433,11 +457,26 @@ __global__ void mean_origin_kernel(const double* __restrict__ pos, const double*
   }
   if (threadIdx.x == 0) {
     const dvec4 r = red[0];
-    const bool ok = r.w != 0.0 && isfinite(r.x / r.w) && isfinite(r.y / r.w) && isfinite(r.z / r.w);
-    origin[0] = ok ? r.x / r.w : 0.0;
-    origin[1] = ok ? r.y / r.w : 0.0;
-    origin[2] = ok ? r.z / r.w : 0.0;
+    const double o0 = r.x / r.w, o1 = r.y / r.w, o2 = r.z / r.w;
+    const bool ok = r.w != 0.0 && isfinite(o0) && isfinite(o1) && isfinite(o2);
+    red[0] = make_dvec4(ok ? o0 : 0.0, ok ? o1 : 0.0, ok ? o2 : 0.0, 0.0);
+    if (blockIdx.x == 0) {
+      bool ne = false;
+      for (int k = 0; k < MO_CHAINS / 32; k++) ne |= differ[k] != 0;
+      const double m0 = mass[0];
+      origin[0] = red[0].x;
+      origin[1] = red[0].y;
+      origin[2] = red[0].z;
+      origin[3] = (!ne && m0 != 0.0 && isfinite(m0)) ? m0 : 0.0;
+    }
   }
+  __syncthreads();
+  const dvec4 o = red[0];
+  const int64_t i = (int64_t)blockIdx.x * MO_CHAINS + threadIdx.x;
+  if (i >= n) return;
+  src[i] = make_float4((float)(pos[3 * i] - o.x), (float)(pos[3 * i + 1] - o.y), (float)(pos[3 * i + 2] - o.z),
+                       (float)mass[i]);
+  lsrc[i] = make_float4((float)lam[3 * i], (float)lam[3 * i + 1], (float)lam[3 * i + 2], 0.f);
 }
 
 // ---------------------------------------------------------------------------
@@ -485,21 +524,33 @@ int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, con
   }
   GH_TRY(ensure(ws.src, (size_t)n * sizeof(float4)));
   GH_TRY(ensure(ws.lsrc, (size_t)n * sizeof(float4)));
-  GH_TRY(ensure(ws.origin, 4 * sizeof(double)));
-  mean_origin_kernel<<<1, 256, 0, st>>>(pos, mass, n, (double*)ws.origin.ptr);
+  GH_TRY(ensure(ws.origin, 4 * sizeof(double) + MO_CHAINS * sizeof(dvec4) + MO_CHAINS / 32 * sizeof(int)));
+  dvec4* chain = (dvec4*)((double*)ws.origin.ptr + 4);
+  int* differ = (int*)(chain + MO_CHAINS);
+  origin_chains_kernel<<<MO_CHAINS / 32, 32, 0, st>>>(pos, mass, n, chain, differ);
   GH_LAUNCH_CHECK();
-  vjp_prepare_mixed_kernel<<<rb, 256, 0, st>>>(pos, mass, lam, n, (const double*)ws.origin.ptr, (float4*)ws.src.ptr,
-                                               (float4*)ws.lsrc.ptr);
+  vjp_prepare_mixed_kernel<<<rb, MO_CHAINS, 0, st>>>(pos, mass, lam, n, chain, differ, (double*)ws.origin.ptr,
+                                                     (float4*)ws.src.ptr, (float4*)ws.lsrc.ptr);
   GH_LAUNCH_CHECK();
-  // Mixed kernel: tiles of VJ_TILE targets, splits of whole VJ_JT-source chunks,
-  // about four resident CTAs per SM, filled twice over.
+  // Mixed kernel: tiles of VJ_TILE targets, splits of whole VJ_JT-source chunks, four
+  // resident CTAs per SM.  Of the splits that fill 1 to 16 waves of CTAs, the one with the
+  // fewest chunks in sequence (half a chunk more per wave for its start): N = 16,384 takes
+  // 19 splits of 7 chunks in one wave, not 32 of 4 in two.  Partial sums up to 64 MB.
   const int64_t mtiles = (n + VJ_TILE - 1) / VJ_TILE;
   const int64_t chunks = (n + VJ_JT - 1) / VJ_JT;
-  int64_t msplits = (8LL * di.num_sms + mtiles - 1) / mtiles;
-  if (msplits > chunks) msplits = chunks;
-  if (msplits < 1) msplits = 1;
-  const int64_t mjlen = ((chunks + msplits - 1) / msplits) * VJ_JT;
-  msplits = (n + mjlen - 1) / mjlen;
+  const int64_t slots = 4LL * di.num_sms;
+  int64_t best = 0, per = chunks;
+  for (int64_t waves = 1; waves <= 16; waves++) {
+    const int64_t most = waves * slots / mtiles;  // splits that fit
+    if (most < 1 || (most > 1 && most * n * 8 * (int64_t)sizeof(float) > (64 << 20))) continue;
+    const int64_t p = (chunks + most - 1) / most, cost = waves * (2 * p + 1);
+    if (best == 0 || cost < best) {
+      best = cost;
+      per = p;
+    }
+  }
+  const int64_t mjlen = per * VJ_JT;
+  const int64_t msplits = (n + mjlen - 1) / mjlen;
   GH_TRY(ensure(ws.part, (size_t)msplits * n * 8 * sizeof(float)));
   prof_begin(st);
   vjp_mixed_kernel<<<dim3((unsigned)mtiles, (unsigned)msplits), VJ_THREADS, 0, st>>>(
@@ -507,8 +558,8 @@ int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, con
       (const double*)ws.origin.ptr + 3);
   prof_end(st);
   GH_LAUNCH_CHECK();
-  vjp_reduce_mixed_kernel<<<rb, 256, 0, st>>>((const float*)ws.part.ptr, (int)msplits, n,
-                                              (const double*)ws.origin.ptr + 3, gpos, gmass);
+  vjp_reduce_mixed_kernel<<<(unsigned)((4 * n + 255) / 256), 256, 0, st>>>(
+      (const float2*)ws.part.ptr, (int)msplits, n, (const double*)ws.origin.ptr + 3, gpos, gmass);
   GH_LAUNCH_CHECK();
   return GH_OK;
 }
