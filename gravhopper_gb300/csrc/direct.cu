@@ -347,6 +347,25 @@ static int launch_mixed(DirectWS& ws, const float4* src, int64_t np, const float
   return GH_OK;
 }
 
+// Targets per CTA of the ordered kernel: the fewest FP64-pipe cycles per source on the SM
+// that holds most CTAs.  A CTA of t targets takes 9 t / 32 warp instructions per source for
+// its pair terms and one, however few of its lanes take part, for its sums.  Force: N = 1500
+// 92 us with 5 against 110 with 4, 2000 153 with 7 against 176 with 4, 4000 496 with 7
+// against 566 with 8; from 6000 on 8 is best (3, 6 and 10 nowhere).
+static int ordered_targets(int64_t nt, int num_sms) {
+  int best = 8;
+  int64_t least = -1;
+  for (const int t : {8, 7, 5, 4, 2}) {
+    const int64_t ctas = (nt + t - 1) / t, per_sm = (ctas + num_sms - 1) / num_sms;
+    const int64_t cost = per_sm * (9 * t + 32);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = t;
+    }
+  }
+  return best;
+}
+
 template <bool SELF, class Epi>
 static int launch_f64(const double* spos, const double* smass, int64_t np, const double* tpos,
                       int64_t nt, double eps, const Epi& epi, cudaStream_t st) {
@@ -355,7 +374,6 @@ static int launch_f64(const double* spos, const double* smass, int64_t np, const
   if (blocks == 0) return GH_OK;
   DeviceInfo di;
   GH_TRY(device_info(&di));
-  const int64_t want = 2LL * di.num_sms;  // CTAs for a full machine
   int form = g_f64_form;
   // The thread-per-target kernel (90 registers, 5 CTAs per SM) fills the machine in
   // whole waves only from about 8 CTAs per SM; below that the CTA-wide kernel is
@@ -365,15 +383,17 @@ static int launch_f64(const double* spos, const double* smass, int64_t np, const
   if (form == 0) {
     direct_f64_kernel<SELF, Epi><<<(unsigned)blocks, F64_THREADS, 0, st>>>(spos, smass, np, tpos, nt,
                                                                            eps * eps, epi);
-  } else if ((nt + 7) / 8 >= want) {
-    direct_f64_ordered_kernel<SELF, 8, Epi>
-        <<<(unsigned)((nt + 7) / 8), F64O_THREADS, 0, st>>>(spos, smass, np, tpos, nt, eps * eps, epi);
-  } else if ((nt + 3) / 4 >= want) {
-    direct_f64_ordered_kernel<SELF, 4, Epi>
-        <<<(unsigned)((nt + 3) / 4), F64O_THREADS, 0, st>>>(spos, smass, np, tpos, nt, eps * eps, epi);
   } else {
-    direct_f64_ordered_kernel<SELF, 2, Epi>
-        <<<(unsigned)((nt + 1) / 2), F64O_THREADS, 0, st>>>(spos, smass, np, tpos, nt, eps * eps, epi);
+    const auto ordered = [&](auto kernel, int tb) {
+      kernel<<<(unsigned)((nt + tb - 1) / tb), F64O_THREADS, 0, st>>>(spos, smass, np, tpos, nt, eps * eps, epi);
+    };
+    switch (ordered_targets(nt, di.num_sms)) {
+      case 2: ordered(direct_f64_ordered_kernel<SELF, 2, Epi>, 2); break;
+      case 4: ordered(direct_f64_ordered_kernel<SELF, 4, Epi>, 4); break;
+      case 5: ordered(direct_f64_ordered_kernel<SELF, 5, Epi>, 5); break;
+      case 7: ordered(direct_f64_ordered_kernel<SELF, 7, Epi>, 7); break;
+      default: ordered(direct_f64_ordered_kernel<SELF, 8, Epi>, 8); break;
+    }
   }
   prof_end(st);
   GH_LAUNCH_CHECK();

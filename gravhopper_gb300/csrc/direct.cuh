@@ -225,7 +225,6 @@ __global__ void __launch_bounds__(F64O_THREADS)
     direct_f64_ordered_kernel(const double* __restrict__ spos, const double* __restrict__ smass, int64_t np,
                               const double* __restrict__ tpos, int64_t nt, double eps2, Epi epi) {
   static_assert(3 * TB <= 32, "the summing lanes form one warp");
-  static_assert(F64O_TERMS % TB == 0, "whole sources per chunk");
   constexpr int JC = F64O_TERMS / TB;  // sources per chunk
   constexpr int JP = JC + 1;           // padded rows: the summing lanes hit distinct banks
   __shared__ dvec4 src[2][JC];
