@@ -305,12 +305,13 @@ __global__ void vjp_reduce_mixed_kernel(const float2* __restrict__ part, int spl
 // takes source (t + k) mod AJ_THREADS at step k and adds the pair's other half to that
 // source's sum in shared memory, a private copy per warp.  The partial sums of rows (part_i)
 // and columns (part_j) are added in a fixed order.
-// Bound by the FP64 pipe: per unordered pair and warp three differences and two DFMAs, 94
-// cycles of an SM as measured, against 296 for its two ordered pairs in a one-sided sum
-// (three differences, three DFMAs of the squared distance, a comparison, a DFMA, each
-// twice); the inverse distance comes from 64-bit fixed point (f64emu.cuh).  N = 65,536:
-// 62.9 -> 20.2 ms; 8192: 996 -> 344 us; 1000: 74 -> 70 us.  Two or four targets per thread:
-// the same from N = 30,000 on, slower below (fewer CTAs).
+// The differences come from 96-bit fixed-point positions and the inverse distance from
+// 64-bit fixed point (f64emu.cuh), about 150 instructions per unordered pair and warp (54
+// cycles of an SM as measured, ALU 71 % busy) with two DFMAs on the FP64 pipe (34 of the
+// cycles).  With FP64 differences it took 94 cycles, and the one-sided sum in FP64 296 (three
+// differences, three DFMAs of the squared distance, a comparison, a DFMA, each twice).
+// N = 65,536: 62.9 -> 20.0 -> 11.7 ms; 8192: 996 -> 364 -> 225 us; 1000: 74 -> 70 -> 56.
+// Two or four targets per thread: the same from N = 30,000 on, slower below (fewer CTAs).
 // ---------------------------------------------------------------------------
 struct PairEps {
   double eps2;
@@ -327,11 +328,28 @@ __device__ __forceinline__ bool pair_inv_distance(double dx, double dy, double d
   return s > 0.0;
 }
 
+// Largest |coordinate|, as the bits of a double (they order like the values).
+__global__ void __launch_bounds__(256)
+    largest_coordinate_kernel(const double* __restrict__ pos, int64_t n3, unsigned long long* __restrict__ out) {
+  unsigned long long m = 0;
+  for (int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x; k < n3; k += (int64_t)gridDim.x * 256) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(pos[k]) & 0x7FFFFFFFFFFFFFFFull;
+    m = b > m ? b : m;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
+    m = q > m ? q : m;
+  }
+  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
 __global__ void __launch_bounds__(AJ_THREADS)
     potential_pairs_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n, double eps2,
-                           int nblocks, int row0, int dlen, double* __restrict__ part_i, double* __restrict__ part_j) {
+                           const unsigned long long* __restrict__ largest, int nblocks, int row0, int dlen,
+                           double* __restrict__ part_i, double* __restrict__ part_j) {
   constexpr int NW = AJ_THREADS / 32;
-  __shared__ dvec4 src[AJ_THREADS];
+  __shared__ uint4 src[3][AJ_THREADS];  // (x, y0), (y1, y2, z0, z1), (z2, -, mass): words of the positions
   __shared__ double col[NW][AJ_THREADS];
   const int tid = threadIdx.x, warp = tid >> 5;
   const int I = row0 + blockIdx.y;
@@ -340,28 +358,49 @@ __global__ void __launch_bounds__(AJ_THREADS)
   PairEps pe;
   pe.eps2 = eps2;
   pe.ok = emu::align_eps2(eps2, pe.E, pe.W);
+  // |x| < 2^E; room: how far the softening's leading bit lies below 2^E
+  const int top = (int)(*largest >> 52), E = top - 1022;
+  const int room = pe.W ? E - (pe.E - 1023) : 1 << 20;
+  const bool fix = pe.ok && (unsigned)(top - 873) <= 300u && room >= 0;
   const int64_t i = (int64_t)I * AJ_THREADS + tid;
-  dvec4 me = make_dvec4(0.0, 0.0, 0.0, 0.0);
-  if (i < n) me = make_dvec4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], mass[i]);
+  const double mass_i = i < n ? mass[i] : 0.0;
+  emu::Fix96 me[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) me[k] = emu::to_fix96(i < n ? pos[3 * i + k] : 0.0, E);
   double phi = 0.0;
   for (int d = d0; d < d1; d++) {
     if (2 * d == nblocks && d > 0 && I >= nblocks / 2) break;  // the lower rows' pairs
     const int J = I + d < nblocks ? I + d : I + d - nblocks;
-    const int64_t j = (int64_t)J * AJ_THREADS + tid;
+    const int64_t j0 = (int64_t)J * AJ_THREADS, j = j0 + tid;
     __syncthreads();
-    if (j < n) src[tid] = make_dvec4(pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], mass[j]);
-    const int jn = i < n ? (int)(n - (j - tid) < AJ_THREADS ? n - (j - tid) : AJ_THREADS) : 0;  // sources to take
+    if (j < n) {
+      emu::Fix96 p[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) p[k] = emu::to_fix96(pos[3 * j + k], E);
+      const uint64_t m = (uint64_t)__double_as_longlong(mass[j]);
+      src[0][tid] = make_uint4(p[0].w[0], p[0].w[1], p[0].w[2], p[1].w[0]);
+      src[1][tid] = make_uint4(p[1].w[1], p[1].w[2], p[2].w[0], p[2].w[1]);
+      src[2][tid] = make_uint4(p[2].w[2], 0u, (uint32_t)m, (uint32_t)(m >> 32));
+    }
+    const int jn = i < n ? (int)(n - j0 < AJ_THREADS ? n - j0 : AJ_THREADS) : 0;  // sources to take
 #pragma unroll
     for (int w = 0; w < NW; w++) col[w][tid] = 0.0;
     __syncthreads();
     for (int k = d ? 0 : 1; k < AJ_THREADS; k++) {  // k = 0 of the block with itself: the particle itself
       const int q = (tid + k) & (AJ_THREADS - 1);
       if (q < jn) {
-        const dvec4 P = src[q];
+        const uint4 A = src[0][q], B = src[1][q], C = src[2][q];
+        const emu::Fix96 p[3] = {{A.x, A.y, A.z}, {A.w, B.x, B.y}, {B.z, B.w, C.x}};
+        const double mass_j = __hiloint2double((int)C.w, (int)C.z);
         double v;
-        if (pair_inv_distance(P.x - me.x, P.y - me.y, P.z - me.z, pe, v)) {
-          phi = fma(-P.w, v, phi);
-          if (d) col[warp][q] = fma(-me.w, v, col[warp][q]);
+        bool add = fix && emu::inv_distance_fix96(p, me, E, room, pe.W, v);
+        if (!add) {
+          const double* x = pos + 3 * (j0 + q);
+          add = pair_inv_distance(x[0] - pos[3 * i], x[1] - pos[3 * i + 1], x[2] - pos[3 * i + 2], pe, v);
+        }
+        if (add) {
+          phi = fma(-mass_j, v, phi);
+          if (d) col[warp][q] = fma(-mass_i, v, col[warp][q]);
         }
       }
       __syncwarp();  // the neighbouring lane takes this source next
@@ -758,10 +797,17 @@ int potential(const double* pos, const double* mass, int64_t n, double eps, doub
     clear_error();
     rows = (rows + 7) / 8;
   }
+  GH_TRY(ensure(ws.origin, sizeof(unsigned long long)));
+  unsigned long long* largest = (unsigned long long*)ws.origin.ptr;
+  GH_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(*largest), st));
+  const int64_t need = (3 * n + 255) / 256, cap = 2LL * di.num_sms;
+  largest_coordinate_kernel<<<(unsigned)(need < cap ? need : cap), 256, 0, st>>>(pos, 3 * n, largest);
+  GH_LAUNCH_CHECK();
   for (int row0 = 0; row0 < nblocks; row0 += (int)rows) {
     const int here = nblocks - row0 < rows ? nblocks - row0 : (int)rows;
-    potential_pairs_kernel<<<dim3((unsigned)splits, (unsigned)here), AJ_THREADS, 0, st>>>(
-        pos, mass, n, eps * eps, nblocks, row0, dlen, (double*)ws.part.ptr, (double*)ws.part_j.ptr);
+    const dim3 grid((unsigned)splits, (unsigned)here);
+    potential_pairs_kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, n, eps * eps, largest, nblocks, row0, dlen,
+                                                        (double*)ws.part.ptr, (double*)ws.part_j.ptr);
     GH_LAUNCH_CHECK();
     potential_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
         (const double*)ws.part.ptr, (const double*)ws.part_j.ptr, n, nblocks, row0, here, (int)splits, phi);

@@ -469,37 +469,139 @@ GH_EMU_HD bool aligned_norm2(double dx, double dy, double dz, int Ee, uint64_t W
   return (unsigned)(E - 873) <= 300u;
 }
 
-// Seed of 1/sqrt(n) as Y0 = y0 2^30 in (2^29, 2^30] to rounding, and the residual h = 1 - n y0^2 as
-// H = h 2^60; false unless |h| < 2^-20.
+// Seed of 1/sqrt(n), n = N10 2^-62, as Y0 = y0 2^30 in (2^29, 2^30], and the residual
+// h = 1 - n y0^2 as H = h 2^60.  The approximation (relative error at most 2^-22.9), the
+// conversion of n and the seed's 23 bits leave |h| < 2^-20; host builds, whose seed may be
+// any, check it.
 GH_EMU_HD bool rsqrt_seed_residual(uint64_t N10, uint32_t& Y0, uint64_t& Y0sq, int64_t& H) {
-  const uint32_t hi = (uint32_t)(N10 >> 32), odd = hi >> 31;  // hi in [2^30, 2^32)
-  const float nf = bitsf((hi >> (7 + odd)) + ((126u + odd) << 23));
-  // y0 in (1/2, 1] plus 1 leaves y0 2^23 in the significand (no conversion instruction)
-  Y0 = (fbits(rsqrt_seed(nf) + 1.0f) - 0x3F800000u) << 7;
+  const uint32_t hi = (uint32_t)(N10 >> 32);
+#ifdef __CUDA_ARCH__
+  const float r = rsqrt_seed(__uint2float_rn(hi));  // y0 2^-15
+  Y0 = (fbits(__fmaf_rn(r, 0x1p15f, 1.0f)) - 0x3F800000u) << 7;
+#else
+  const float r = rsqrt_seed((float)hi);
+  Y0 = (fbits(fmaf(r, 0x1p15f, 1.0f)) - 0x3F800000u) << 7;
+#endif
   Y0sq = (uint64_t)Y0 * Y0;  // y0^2 2^60, at most a little above 2^60
   H = (int64_t)((1ull << 60) - umulhi_low(N10, Y0sq << 2));
+#ifdef __CUDA_ARCH__
+  return true;
+#else
   return (uint64_t)(H + (1ll << 40)) < (1ull << 41);
+#endif
+}
+
+// h^2 2^68 of H = h 2^60, |h| < 2^-20.
+GH_EMU_HD uint32_t residual_square(int64_t H) {
+  const int32_t h = (int32_t)(H >> 10);
+#ifdef __CUDA_ARCH__
+  return (uint32_t)__mulhi(h, h);
+#else
+  return (uint32_t)(((int64_t)h * h) >> 32);
+#endif
+}
+
+// a (1 + c) for a = A 2^32 and c = C 2^-64, |C| < 2^45 (short by at most 1).
+GH_EMU_HD uint64_t scale_up(uint32_t A, int64_t C) {
+  const int32_t ch = (int32_t)(C >> 32);
+  const uint32_t cl = (uint32_t)C;
+  return (((uint64_t)A << 32) | (uint32_t)(((uint64_t)A * cl) >> 32)) + (uint64_t)((int64_t)(int32_t)A * ch);
+}
+
+// 1/sqrt(s), s = n 4^e, n = N10 2^-62, rounded once; false when the seed check fails.
+GH_EMU_HD bool inv_root_rn(uint64_t N10, int e, double& out) {
+  uint64_t Y0sq;
+  uint32_t Y0;
+  int64_t H;
+  if (!rsqrt_seed_residual(N10, Y0, Y0sq, H)) return false;
+  // y = y0 (1 + c), c = h (1/2 + 3/8 h) as C = c 2^64; the next term is below 2^-61
+  const int64_t C = (H << 3) + (int64_t)((3 * residual_square(H)) >> 7);
+  const uint64_t Y = scale_up(Y0, C);        // y 2^62, in [2^61, 2^62] to rounding
+  const uint64_t mant = (Y + 256) >> 9;      // in [2^52, 2^53]; 2^53 carries into the exponent
+  out = bitsd(((uint64_t)(1021 - e) << 52) + mant);  // s^(-1/2) = y 2^-e
+  return true;
 }
 
 // 1/sqrt(dx^2 + dy^2 + dz^2 + eps^2), rounded once (the potential's pairs); false outside
 // the range of aligned_norm2.
 GH_EMU_HD bool inv_distance(double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
-  uint64_t N10, Y0sq;
-  uint32_t Y0;
-  int64_t H;
+  uint64_t N10;
   int e;
-  bool ok = aligned_norm2(dx, dy, dz, Ee, W, N10, e);
-  ok &= rsqrt_seed_residual(N10, Y0, Y0sq, H);
-  if (!ok) return false;
-  // y 2^62 = y0 2^62 (1 + c), c = h (1/2 + 3/8 h) as C = c 2^60; the next term is below 2^-61
-  const int32_t h = (int32_t)(H >> 10);  // h 2^50
-  const int64_t C = (H >> 1) + ((((int64_t)h * h >> 20) * 3) >> 23);
-  const uint64_t y0 = (uint64_t)Y0 << 32;
-  const uint64_t Y = y0 + (uint64_t)(smulhi_low(y0, C << 22) >> 18);  // in [2^61, 2^62] to rounding
-  const int up = (int)(Y >> 62);
-  const uint64_t mant = (Y >> (9 + up)) + ((Y >> (8 + up)) & 1);  // in [2^52, 2^53]
-  out = bitsd(((uint64_t)(up - 53 - e + 1074) << 52) + mant);  // s^(-1/2) = y 2^-e
-  return true;
+  return aligned_norm2(dx, dy, dz, Ee, W, N10, e) & inv_root_rn(N10, e, out);
+}
+
+// Positions in 96-bit two's complement fixed point, unit 2^(E - 94) for |x| < 2^E: exact for
+// |x| >= 2^(E - 42), truncated below, so a difference is off by less than two units.
+struct Fix96 {
+  uint32_t w[3];
+};
+GH_EMU_HD Fix96 to_fix96(double x, int E) {
+  const uint64_t b = dbits(x);
+  const int ex = (int)(b >> 52) & 0x7FF;
+  const uint64_t M = ex ? (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull : 0;
+  const int sh = (ex - 1075) - (E - 94);  // <= 41
+  const uint64_t lo = sh >= 0 ? M << sh : shr_clamp(M, -sh);
+  const uint32_t hi = sh > 0 ? (uint32_t)(M >> (64 - sh)) : 0u;
+  const uint64_t neg = (uint64_t)0 - (b >> 63);  // all ones when negative: ~v + 1
+  const uint64_t l2 = (lo ^ neg) + (b >> 63);
+  Fix96 r;
+  r.w[0] = (uint32_t)l2;
+  r.w[1] = (uint32_t)(l2 >> 32);
+  r.w[2] = (hi ^ (uint32_t)neg) + (uint32_t)((b >> 63) & (l2 == 0));
+  return r;
+}
+
+// |a - b| in 96 bits (one unit short of it when negative).
+GH_EMU_HD void fix96_distance(const Fix96& a, const Fix96& b, uint32_t& d0, uint32_t& d1, uint32_t& d2) {
+#ifdef __CUDA_ARCH__
+  asm("sub.cc.u32 %0, %3, %6;\n\tsubc.cc.u32 %1, %4, %7;\n\tsubc.u32 %2, %5, %8;"
+      : "=r"(d0), "=r"(d1), "=r"(d2)
+      : "r"(a.w[0]), "r"(a.w[1]), "r"(a.w[2]), "r"(b.w[0]), "r"(b.w[1]), "r"(b.w[2]));
+#else
+  const uint64_t al = ((uint64_t)a.w[1] << 32) | a.w[0], bl = ((uint64_t)b.w[1] << 32) | b.w[0], dl = al - bl;
+  d0 = (uint32_t)dl;
+  d1 = (uint32_t)(dl >> 32);
+  d2 = a.w[2] - b.w[2] - (al < bl);
+#endif
+  const uint32_t s = (uint32_t)((int32_t)d2 >> 31);
+  d0 ^= s;
+  d1 ^= s;
+  d2 ^= s;
+}
+
+GH_EMU_HD uint32_t shl_funnel(uint32_t lo, uint32_t hi, int s) {  // 0 <= s <= 31
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, s);
+#else
+  return s ? (hi << s) | (lo >> (32 - s)) : hi;
+#endif
+}
+
+GH_EMU_HD int clz32(uint32_t v) {
+#ifdef __CUDA_ARCH__
+  return __clz((int)v);
+#else
+  return v ? __builtin_clz(v) : 32;
+#endif
+}
+
+// inv_distance of two fixed-point positions, without a floating-point difference.  e_eps
+// and W as align_eps2 gives them (e_eps = Ee - 1023), room = E - e_eps >= 0 (a large number
+// for eps = 0): the squares are aligned at the largest difference's leading bit, or at the
+// softening's.  False when both lie below 2^(E - 32).
+GH_EMU_HD bool inv_distance_fix96(const Fix96* a, const Fix96* b, int E, int room, uint64_t W, double& out) {
+  uint32_t x0, x1, x2, y0, y1, y2, z0, z1, z2;
+  fix96_distance(a[0], b[0], x0, x1, x2);
+  fix96_distance(a[1], b[1], y0, y1, y2);
+  fix96_distance(a[2], b[2], z0, z1, z2);
+  int sh = clz32(x2 | y2 | z2) - 1;  // in [0, 31]
+  sh = room < sh ? room : sh;
+  const uint64_t X = ((uint64_t)shl_funnel(x1, x2, sh) << 32) | shl_funnel(x0, x1, sh);
+  const uint64_t Y = ((uint64_t)shl_funnel(y1, y2, sh) << 32) | shl_funnel(y0, y1, sh);
+  const uint64_t Z = ((uint64_t)shl_funnel(z1, z2, sh) << 32) | shl_funnel(z0, z1, sh);
+  const uint64_t S = square_hi(X) + square_hi(Y) + square_hi(Z) + shr_clamp(W, 2 * (room - sh));
+  const int big = (S >> 62) != 0;
+  return ((S >> 59) != 0) & inv_root_rn(big ? S : S << 2, E - sh + big, out);
 }
 
 GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
@@ -513,11 +615,10 @@ GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, 
   ok &= (unsigned)(Em - 523) <= 1000u;  // |m| in [2^-500, 2^501)
   ok &= rsqrt_seed_residual(N10, Y0, Y0sq, H);
   if (!ok) return false;
-  // y0^3 2^61, then times 1 + c, c = h (3/2 + 15/8 h) as C = c 2^60, |C| < 2^41
+  // y0^3 2^61, then times 1 + c, c = h (3/2 + 15/8 h) as C = c 2^64, |C| < 2^45
   const uint64_t Y3 = umulhi_low(Y0sq << 2, (uint64_t)Y0 << 33);
-  const int32_t h = (int32_t)(H >> 10);  // h 2^50
-  const int64_t C = H + (H >> 1) + ((((int64_t)h * h >> 20) * 15) >> 23);
-  const uint64_t F = Y3 + (uint64_t)(smulhi_low(Y3, C << 22) >> 18);
+  const int64_t C = H * 24 + (int64_t)((15 * (uint64_t)residual_square(H)) >> 7);
+  const uint64_t F = Y3 + (uint64_t)(smulhi_low(Y3, C));
   // times the mass's significand mm in [1, 2): T0 = mm y^3 2^62 in [2^59, 2^63]
   const uint64_t T0 = umulhi_low(F << 2, ((bm & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << 11);
   const int lz = clz64(T0);
