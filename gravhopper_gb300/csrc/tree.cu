@@ -1194,8 +1194,13 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
 
 // How a walk is split over warps: `segs` warps per 32 targets, each walking one range of
 // the preorder.  Targets that have a place of their own in it (particles, sorted points)
-// visit about as many cells in each doubling of the distance from that place, so the
-// ranges grow geometrically with it; 32 unsorted points are anywhere, so theirs are equal.
+// open cells that are near them in space: those of d nodes around that place and, beyond,
+// the ones that lie along the faces of larger cells, whose number grows like the faces'
+// area, d^(2/3).  So the ranges are equal in the 2/3 power of the distance from that place
+// (equal in its logarithm, the far ranges held up to 17 times the average's steps: force
+// 664 us at N = 16,384 against 575, and equal ranges 630).  Just two meet next to the
+// place, where they are equal in the logarithm (262,144: 4.66 -> 4.59 ms).  32 unsorted
+// points are anywhere, so theirs are equal.
 struct WalkSplit {
   int segs;
   double* part;           // [group][seg][component][lane] partial sums
@@ -1206,6 +1211,7 @@ struct WalkSplit {
   int64_t n;
 };
 constexpr float TW_SEG_NEAR = 128.f;  // nodes around its own place that a group visits densely
+constexpr float TW_SEG_POWER = 2.f / 3.f;
 
 // Place in the preorder of target slot q.
 __device__ __forceinline__ int walk_own(const WalkSplit& sp, int64_t q, int64_t nt, int nnodes) {
@@ -1224,14 +1230,24 @@ __device__ __forceinline__ int walk_own(const WalkSplit& sp, int64_t q, int64_t 
 }
 
 // First node of segment s (of K) for a group whose own place is node `own` (-1: none).
+// Never falls with s: steps of u are 2e-5 and more, __powf is good to 1e-6 there.
 __device__ __forceinline__ int walk_bound(int s, int K, int own, int nnodes) {
   if (s <= 0) return 0;
   if (s >= K) return nnodes;
   if (own < 0) return (int)((int64_t)nnodes * s / K);
-  const float left = log2f(1.f + (float)own / TW_SEG_NEAR), right = log2f(1.f + (float)(nnodes - own) / TW_SEG_NEAR);
-  const float u = (left + right) * (float)s / (float)K;
-  const float d = TW_SEG_NEAR * (exp2f(fabsf(u - left)) - 1.f);
-  const int b = u < left ? own - (int)d : own + (int)d;
+  const float l = 1.f + (float)own / TW_SEG_NEAR, r = 1.f + (float)(nnodes - own) / TW_SEG_NEAR;
+  float d;
+  bool before;
+  if (K == 2) {
+    before = l > r;
+    d = sqrtf(before ? l / r : r / l) - 1.f;
+  } else {
+    const float left = __powf(l, TW_SEG_POWER) - 1.f, right = __powf(r, TW_SEG_POWER) - 1.f;
+    const float u = (left + right) * (float)s / (float)K - left;
+    before = u < 0.f;
+    d = __powf(1.f + fabsf(u), 1.f / TW_SEG_POWER) - 1.f;
+  }
+  const int b = before ? own - (int)(TW_SEG_NEAR * d) : own + (int)(TW_SEG_NEAR * d);
   return b < 0 ? 0 : (b > nnodes ? nnodes : b);
 }
 
@@ -1672,19 +1688,19 @@ static Buffer g_stats[64];
 // a chain of dependent steps, so a walk with fewer groups than the GPU holds warps
 // (36 per SM) takes as long as its longest chain; splitting the chains fills the GPU, at
 // about 2 % more steps per doubling (the ancestors of each segment's first cell).
-// Up to 1024 groups some 28,000 warps in all were fastest, at most 64 per group (256 for
-// unsorted points, whose walks have no dense part); above, three warps per group below
-// 2048 groups, two up to 12,288 (3/4 of the machine's warps and more were slower split
-// further).  Force, unsplit -> split, theta 0.7: N = 2000 Plummer 770 -> 314 us, 8000
-// 1001 -> 486; Hernquist + disk 16,384 1376 -> 707, 60,013 1945 -> 1421, 131,072 2698 ->
-// 2618, 262,144 4978 -> 4716; at 1,048,576 two warps would cost 18.7 -> 19.1 ms.  Points
-// in a 250,000-particle system, theta 0.5: 100 unsorted 17.6 -> 0.9 ms, 8100 17.9 -> 3.0,
-// 30,011 sorted 6.4 -> 3.6.
-static int walk_segments(int64_t groups, bool placed) {
+// All in all 14,000 warps and n / 5 more were fastest (a larger tree has more steps to
+// share), at most 64 per group of particles, 128 of sorted points and 256 of unsorted ones.
+// Less than 12 for each of many groups is worse than two, and 3/8 of a million targets
+// fill the GPU unsplit.  Force, unsplit -> split, theta 0.7: N = 500 Plummer 302 -> 96 us,
+// 2000 577 -> 131, 8000 840 -> 303; Hernquist + disk 16,384 1304 -> 575, 30,000 1541 ->
+// 842, 60,013 1835 -> 1375, 131,072 2580 -> 2540, 262,144 4847 -> 4590; at 1,048,576 two
+// warps would cost 18.7 -> 19.1 ms.  Points in a 250,000-particle system, theta 0.5: 100
+// unsorted 17.6 -> 0.85 ms, 8100 16.9 -> 2.9, 10,000 sorted 7.0 -> 1.8, 30,011 6.0 -> 2.8,
+// 100,000 6.3 -> 5.5.
+static int walk_segments(int64_t groups, int64_t n, int cap) {
   if (groups > 12288) return 1;
-  if (groups >= 2048) return 2;
-  if (groups > 1024) return 3;
-  const int64_t cap = placed ? 64 : 256, k = 28672 / groups;
+  const int64_t warps = 14000 + (n < 262144 ? n : 262144) / 5, k = warps / groups;
+  if (k < 12 && groups > 2816) return 2;
   return (int)(k < cap ? k : cap);
 }
 
@@ -1694,9 +1710,9 @@ static int launch_walk_f64(TreeWS& ws, const NodeArrays& na, const BuiltTree& bt
                            const Epi& epi, unsigned long long* stats, cudaStream_t st) {
   const int64_t groups = (nt + 31) / 32;
   WalkSplit sp = {};
-  sp.segs = stats ? 1 : walk_segments(groups, self || order);  // the counters are those of whole walks
+  sp.segs = stats ? 1 : walk_segments(groups, bt.n, self ? 64 : (order ? 128 : 256));  // the counters are those of whole walks
   const size_t cb = (size_t)groups * sizeof(int);
-  if (sp.segs > 1) {  // at most 22 MB of scratch; without it the walk is not split
+  if (sp.segs > 1) {  // at most 51 MB of scratch; without it the walk is not split
     int rc = ensure(ws.wpart, (size_t)groups * sp.segs * 96 * sizeof(double));
     if (rc == GH_OK && ws.wcount.bytes < cb) ws.wcount_zeroed = 0;
     if (rc == GH_OK) rc = ensure(ws.wcount, cb);

@@ -38,8 +38,8 @@ def test_signs_and_sizes_of_masses(lib, cuda):
     check(_jbgrav.tree_force(ic["pos"], mass, 0.05, 0.0), oracle.tree_force(ic["pos"], mass, 0.05, 0.0))
 
 
-# groups of 32 targets: 1, 2, 5, 63, 1024, 1025 (three warps each), 2048 (two)
-@pytest.mark.parametrize("n", [1, 2, 32, 33, 129, 2000, 32768, 32769, 65536])
+# groups of 32 targets: 1, 2, 5, 63, 1024, 1025, 2048, 2816 (11 warps each), 2817 (two)
+@pytest.mark.parametrize("n", [1, 2, 32, 33, 129, 2000, 32768, 32769, 65536, 90112, 90113])
 def test_particles(lib, cuda, n):
     from gravhopper_gb300 import _jbgrav, ics
     ic = ics.hernquist_disk(n, seed=7)
@@ -50,7 +50,7 @@ def test_particles(lib, cuda, n):
 
 # 8191 points keep their order, from 8192 they are sorted; 1 and 2 particles: every range
 # but one is empty
-@pytest.mark.parametrize("n,points", [(3000, 1), (3000, 31), (3000, 33), (3000, 8191), (3000, 8192), (3000, 33000),
+@pytest.mark.parametrize("n,points", [(3000, 1), (3000, 31), (3000, 33), (3000, 8191), (3000, 8192), (3000, 33000), (3000, 90113),
                                       (1, 40), (2, 9000)])
 def test_points(lib, cuda, n, points):
     from gravhopper_gb300 import _jbgrav, ics
