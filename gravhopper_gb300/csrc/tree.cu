@@ -1059,26 +1059,39 @@ __device__ __forceinline__ void walk_offset(const WalkTarget& T, const float4& A
   dz = (A.z - T.h2) + (Lo.z - T.l2);
 }
 
-// The opening test of an internal cell: accepted when size / distance < theta, decided in
-// FP32 outside the margins, else with the reference's FP64 operations (exact counts those).
-__device__ __forceinline__ bool walk_accept(const WalkTarget& T, f2 dxy, float dz, float s2, float th2_lo, float th2_hi,
-                                            const dvec4* __restrict__ nC, int node, double p0, double p1, double p2,
-                                            double theta, unsigned& exact) {
-  float dx, dy;
-  f2split(dxy, dx, dy);
-  const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-  // d2 = inf (overflow) accepts, as the exact test does for so distant a cell
-  const bool usable = d2 > T.near2;
-  if (usable && s2 < th2_lo * d2) return true;
-  if (usable && s2 > th2_hi * d2) return false;
-  // gravoct_calc_accel opening test with the reference's FP64 operations
-  exact++;
+// gravoct_calc_accel's opening test with the reference's FP64 operations, on the target's
+// position, which pos(p0, p1, p2) gives.  Rare, and a call: inline, its division and square
+// root took the registers and the branches of every step.
+template <class Pos>
+__device__ __noinline__ bool walk_exact(const dvec4* __restrict__ nC, int node, Pos pos, double theta) {
+  double p0, p1, p2;
+  pos(p0, p1, p2);
   const dvec4 C = nC[node];
   const double e0 = dsub(C.x, p0), e1 = dsub(C.y, p1), e2 = dsub(C.z, p2);
   double nd = dmul(e0, e0);
   nd = dadd(nd, dmul(e1, e1));
   nd = dadd(nd, dmul(e2, e2));
   return ddiv(C.w, dsqrt(nd)) < theta;
+}
+
+// Whether a visited cell is accepted: a leaf always, another when size / distance < theta,
+// decided in FP32 outside the margins, else exactly (exact counts those).  One branch, the
+// rare one: the rest is predicates.
+template <class Pos>
+__device__ __forceinline__ bool walk_accept(const WalkTarget& T, f2 dxy, float dz, float s2, bool leaf, bool visit,
+                                            float th2_lo, float th2_hi, const dvec4* __restrict__ nC, int node,
+                                            const Pos& pos, double theta, unsigned& exact) {
+  float dx, dy;
+  f2split(dxy, dx, dy);
+  const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+  // d2 = inf (overflow) accepts, as the exact test does for so distant a cell
+  const bool usable = d2 > T.near2;
+  bool accept = leaf | (usable & (s2 < th2_lo * d2));
+  if (visit & !accept & !(usable & (s2 > th2_hi * d2))) {
+    exact++;
+    accept = walk_exact(nC, node, pos, theta);
+  }
+  return accept & visit;
 }
 
 // Walk counters of a warp into stats.
@@ -1105,6 +1118,15 @@ __device__ __forceinline__ bool walk_is_chain(const WalkRec* __restrict__ nR, in
   return nxt != node + 1 && node + 1 < nnodes && __float_as_int(nR[node + 1].L.w) == nxt;
 }
 
+// Mixed walk.  A step is a chain (record, opening test, the lanes' next node) of some 50
+// instructions, and at 62 % of the issue slots the instructions set the time: so a step has
+// one branch, for the rare exact test, its interaction is formed by every lane, the fold
+// is a loop of its own around the steps, and the position for the exact test is read again
+// instead of held.  N = 16,384 theta 0.7 408 -> 318 us, 60,013 505 -> 399, 1,048,576 theta
+// 0.5 9.62 -> 8.49 ms (the FP64 walk, whose steps also end in rounds of interactions: 344 ->
+// 322 us, 1141 -> 1085, 17.34 -> 17.20 ms at theta 0.7).  More warps with fewer registers
+// (spills), the next record's load ahead of the interaction, and votes in place of the
+// minimum were all slower.
 template <bool GUARD, bool STATS, class Epi>
 __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     tree_walk_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, const int* __restrict__ nodes,
@@ -1115,62 +1137,61 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
   if (nnodes == 0) return;  // a build that did not succeed
   const int64_t slot = (int64_t)blockIdx.x * TW_THREADS + threadIdx.x;
   const bool valid = slot < nt;
-  const int64_t t = valid ? (order ? (int64_t)order[slot] : slot) : 0;
-  double p0 = 0.0, p1 = 0.0, p2 = 0.0;
-  if (valid) {
+  const auto pos = [=](double& p0, double& p1, double& p2) {  // read again by the exact test
+    const int64_t t = order ? (int64_t)order[slot] : slot;
     p0 = tpos[3 * t];
     p1 = tpos[3 * t + 1];
     p2 = tpos[3 * t + 2];
-  }
+  };
+  double p0 = 0.0, p1 = 0.0, p2 = 0.0;
+  if (valid) pos(p0, p1, p2);
   const WalkTarget T = walk_target(p0, p1, p2);
   const float eps2f = (float)eps2;
   float px = 0.f, py = 0.f, pz = 0.f;                                // FP32 partial
   float hx = 0.f, hy = 0.f, hz = 0.f, qx = 0.f, qy = 0.f, qz = 0.f;  // two-sum hi, lo
-  int pending = 0;
   unsigned n_step = 0, n_visit = 0, n_inter = 0, n_exact = 0, n_leaf = 0, n_chain = 0;  // walk counters (STATS)
   int skip = valid ? 0 : 0x7fffffff;
   int node = __reduce_min_sync(0xffffffffu, skip);
   while (node < nnodes) {
-    if (STATS) {
-      n_step++;
-      n_chain += walk_is_chain(nR, node, nnodes);
-    }
-    int lane_next = skip;
-    if (node >= skip) {
-      if (STATS) n_visit++;
+    int left = TW_FOLD;
+    do {
+      if (STATS) {
+        n_step++;
+        n_chain += walk_is_chain(nR, node, nnodes);
+      }
       const float4 A = nR[node].A;
       const float4 Lo = nR[node].L;
-      const float4 O = nR[node].O;  // loaded with the rest of the record: most visits are accepted
+      const float4 O = nR[node].O;
       const int nx = __float_as_int(Lo.w);
-      bool accept = (nx == node + 1);  // leaf
+      const bool visit = node >= skip, leaf = nx == node + 1;
       f2 dxy;
       float dz;
       walk_offset(T, A, Lo, dxy, dz);
-      if (!accept) accept = walk_accept(T, dxy, dz, A.w, th2_lo, th2_hi, nC, node, p0, p1, p2, theta, n_exact);
+      const bool accept = walk_accept(T, dxy, dz, A.w, leaf, visit, th2_lo, th2_hi, nC, node, pos, theta, n_exact);
+      if (STATS) {
+        n_visit += visit;
+        n_inter += accept;
+        n_leaf += accept && leaf;
+      }
+      // formed by every lane, added where accepted: no branch
+      float ex, ey;
+      f2split(f2add(dxy, f2make(O.x, O.y)), ex, ey);
+      const float ez = dz + O.z;
+      const float s = fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, eps2f)));
+      float r = rsqrt_approx(s);
+      if (GUARD) r = s > 0.f ? r : 0.f;
+      const float f = O.w * (r * (r * r));
       if (accept) {
-        if (STATS) {
-          n_inter++;
-          if (nx == node + 1) n_leaf++;
-        }
-        float ex, ey;
-        f2split(f2add(dxy, f2make(O.x, O.y)), ex, ey);
-        const float ez = dz + O.z;
-        const float s = fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, eps2f)));
-        float r = rsqrt_approx(s);
-        if (GUARD) r = s > 0.f ? r : 0.f;
-        const float f = O.w * (r * (r * r));
         px = fmaf(f, ex, px);
         py = fmaf(f, ey, py);
         pz = fmaf(f, ez, pz);
         skip = nx;
-        lane_next = nx;
-      } else {
-        lane_next = node + 1;
       }
-    }
+      node = __reduce_min_sync(0xffffffffu, visit & !accept ? node + 1 : skip);
+    } while (--left && node < nnodes);
     // fold the FP32 partials every TW_FOLD warp steps (at most one interaction per
-    // target per step): a warp-uniform branch
-    if (++pending == TW_FOLD) {
+    // target per step); what is left of them at the end is added as it is
+    if (left == 0) {
       float sx, ex;
       two_sum(hx, px, sx, ex);
       hx = sx;
@@ -1182,13 +1203,11 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
       hz = sx;
       qz += ex;
       px = py = pz = 0.f;
-      pending = 0;
     }
-    node = __reduce_min_sync(0xffffffffu, lane_next);
   }
   if (STATS) walk_count(stats, n_step, n_visit, n_inter, n_exact, n_leaf, n_chain);
   if (valid)
-    epi(t, (double)hx + (double)qx + (double)px, (double)hy + (double)qy + (double)py,
+    epi(order ? (int64_t)order[slot] : slot, (double)hx + (double)qx + (double)px, (double)hy + (double)qy + (double)py,
         (double)hz + (double)qz + (double)pz);
 }
 
@@ -1279,6 +1298,11 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     p1 = tpos[3 * t + 1];
     p2 = tpos[3 * t + 2];
   }
+  const auto pos = [=](double& a0, double& a1, double& a2) {
+    a0 = p0;
+    a1 = p1;
+    a2 = p2;
+  };
   WalkTarget T = walk_target(p0, p1, p2);
   // keeps the compiler from forming the residuals again inside the loop to save registers,
   // where each is three FP64-pipe instructions (one residual per interaction was: 29.0
@@ -1311,7 +1335,7 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
         float dz;
         const float4 A = nR[c].A;
         walk_offset(T, A, Lo, dxy, dz);
-        if (walk_accept(T, dxy, dz, A.w, th2_lo, th2_hi, nC, c, p0, p1, p2, theta, n_exact)) skip = nx;
+        if (walk_accept(T, dxy, dz, A.w, false, true, th2_lo, th2_hi, nC, c, pos, theta, n_exact)) skip = nx;
       }
       c++;
     }
@@ -1323,32 +1347,25 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
       n_step++;
       n_chain += walk_is_chain(nR, node, nnodes);
     }
-    int lane_next = skip;
-    if (node >= skip) {
-      if (STATS) n_visit++;
-      const float4 A = nR[node].A;
-      const float4 Lo = nR[node].L;
-      const int nx = __float_as_int(Lo.w);
-      bool accept = (nx == node + 1);  // leaf
-      if (!accept) {
-        f2 dxy;
-        float dz;
-        walk_offset(T, A, Lo, dxy, dz);
-        accept = walk_accept(T, dxy, dz, A.w, th2_lo, th2_hi, nC, node, p0, p1, p2, theta, n_exact);
-      }
-      if (accept) {
-        if (STATS) {
-          n_inter++;
-          if (nx == node + 1) n_leaf++;
-        }
-        fq[(fq_head + fq_n) & (TW_FQ - 1)][threadIdx.x] = node;  // evaluated in a later round
-        fq_n++;
-        skip = nx;
-        lane_next = nx;
-      } else {
-        lane_next = node + 1;
-      }
+    const float4 A = nR[node].A;
+    const float4 Lo = nR[node].L;
+    const int nx = __float_as_int(Lo.w);
+    const bool visit = node >= skip, leaf = nx == node + 1;
+    f2 dxy;
+    float dz;
+    walk_offset(T, A, Lo, dxy, dz);
+    const bool accept = walk_accept(T, dxy, dz, A.w, leaf, visit, th2_lo, th2_hi, nC, node, pos, theta, n_exact);
+    if (STATS) {
+      n_visit += visit;
+      n_inter += accept;
+      n_leaf += accept && leaf;
     }
+    if (accept) {
+      fq[(fq_head + fq_n) & (TW_FQ - 1)][threadIdx.x] = node;  // evaluated in a later round
+      fq_n++;
+      skip = nx;
+    }
+    const int lane_next = visit & !accept ? node + 1 : skip;
     // a round of FP64 interactions when enough lanes have one waiting; a FIFO that
     // just became full forces one, so a FIFO never holds more than TW_FQ
     const unsigned waiting = __ballot_sync(0xffffffffu, fq_n > 0);
