@@ -38,8 +38,9 @@ def test_signs_and_sizes_of_masses(lib, cuda):
     check(_jbgrav.tree_force(ic["pos"], mass, 0.05, 0.0), oracle.tree_force(ic["pos"], mass, 0.05, 0.0))
 
 
+# 8193: no small build, 8704 and 8705: tiles of 512 in the moments' sums
 # groups of 32 targets: 1, 2, 5, 63, 1024, 1025, 2048, 2816 (11 warps each), 2817 (two)
-@pytest.mark.parametrize("n", [1, 2, 32, 33, 129, 2000, 32768, 32769, 65536, 90112, 90113])
+@pytest.mark.parametrize("n", [1, 2, 32, 33, 129, 2000, 8193, 8704, 8705, 32768, 32769, 65536, 90112, 90113])
 def test_particles(lib, cuda, n):
     from gravhopper_gb300 import _jbgrav, ics
     ic = ics.hernquist_disk(n, seed=7)
