@@ -6,12 +6,12 @@
 //   dL/dx_k = sum_{j != k} [ q u - p (d.u) d ],   u = m_k lambda_j - m_j lambda_k,
 //             q = s^{-3/2}, p = 3 s^{-5/2}   (the softened tidal tensor applied to u)
 //   dL/dm_k = - sum_{j != k} q (lambda_j . d)
-// Potential: phi_k = - sum_{j != k} m_j s^{-1/2}.
+// Potential: phi_k = - sum_{j != k} m_j s^{-1/2}, each unordered pair once.
 //
-// Work split (VJP): a 2-D grid of (target tile, source split); each CTA writes per-target
-// partial sums for its split to scratch and a reduction kernel adds the splits in
-// split order, so results do not depend on scheduling.  FP64: one thread per target,
-// s^{-1/2} from the hardware approximation refined by two Newton steps.  Mixed: FP32
+// Work split (mixed VJP): a 2-D grid of (target tile, source split); each CTA writes
+// per-target partial sums for its split to scratch and a reduction kernel adds the splits
+// in split order, so results do not depend on scheduling.  FP64 VJP and potential: each
+// unordered pair of blocks in one CTA, its sums likewise reduced in a fixed order.  Mixed: FP32
 // pair arithmetic on coordinates relative to the mass-weighted centre, per-chunk FP32
 // partials folded into two-sum (hi, lo) accumulators, FP64 reduction.
 #include <mutex>
@@ -35,57 +35,96 @@ __device__ __forceinline__ double rsqrt_nr(double s) {
 }
 
 // ---------------------------------------------------------------------------
-// FP64 VJP: part[(split*n + k)*4 + {0,1,2,3}] = (gx, gy, gz, gm)
+// FP64 VJP.  A pair's term of dL/dx changes sign with the order of its particles, so each
+// unordered pair is taken once: row I of AJ_THREADS targets meets blocks I .. I + nblocks/2
+// (cyclic; of two opposite blocks only the lower row takes the pairs), a warp's lanes at
+// different sources of a block, whose sums wait in shared memory, one set per warp.  Where that is few
+// CTAs, `parts` of them share a pair of blocks.
+// FP64-pipe bound: 38 operations per unordered pair against 2 x 28 with ordered ones (per
+// VJP, N = 500 160 -> 39 us, 2000 253 -> 184, 4096 877 -> 625, 16,384 13.08 -> 8.97 ms).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(AJ_THREADS)
-    vjp_f64_kernel(const double* __restrict__ pos, const double* __restrict__ mass, const double* __restrict__ lam,
-                   int64_t n, double eps2, int64_t jlen, double* __restrict__ part) {
-  __shared__ dvec4 sp[AJ_THREADS], sl[AJ_THREADS];
-  const int64_t k = (int64_t)blockIdx.x * AJ_THREADS + threadIdx.x;
-  const int64_t split = blockIdx.y;
-  const int64_t j0 = split * jlen, j1 = (j0 + jlen) < n ? j0 + jlen : n;
-  const bool valid = k < n;
-  const int64_t kk = valid ? k : 0;
-  const double xk = pos[3 * kk], yk = pos[3 * kk + 1], zk = pos[3 * kk + 2], mk = mass[kk];
-  const double lxk = lam[3 * kk], lyk = lam[3 * kk + 1], lzk = lam[3 * kk + 2];
+    vjp_pairs_f64_kernel(const double* __restrict__ pos, const double* __restrict__ mass,
+                         const double* __restrict__ lam, int64_t n, double eps2, int nblocks, int row0, int parts, int len,
+                         double* __restrict__ part_i, double* __restrict__ part_j) {
+  constexpr int NW = AJ_THREADS / 32;
+  __shared__ double src[7][AJ_THREADS];  // x, y, z, mass, lambda
+  __shared__ double col[NW][4][AJ_THREADS];
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int I = row0 + blockIdx.y;
+  const int dmax = nblocks / 2;
+  const int end = (dmax + 1) * parts, e0 = blockIdx.x * len, e1 = e0 + len < end ? e0 + len : end;
+  const int64_t i = (int64_t)I * AJ_THREADS + tid, ii = i < n ? i : 0;
+  const double xi = pos[3 * ii], yi = pos[3 * ii + 1], zi = pos[3 * ii + 2], mi = mass[ii];
+  const double lxi = lam[3 * ii], lyi = lam[3 * ii + 1], lzi = lam[3 * ii + 2];
   double gx = 0.0, gy = 0.0, gz = 0.0, gm = 0.0;
-  for (int64_t c = j0; c < j1; c += AJ_THREADS) {
+  for (int e = e0; e < e1; e++) {
+    const int d = e / parts, k0 = (e - d * parts) * (AJ_THREADS / parts), k1 = k0 + AJ_THREADS / parts;
+    if (2 * d == nblocks && d > 0 && I >= nblocks / 2) break;  // the lower rows' pairs
+    const int J = I + d < nblocks ? I + d : I + d - nblocks;
+    const int64_t j0 = (int64_t)J * AJ_THREADS, j = j0 + tid;
     __syncthreads();
-    const int64_t j = c + threadIdx.x;
-    if (j < j1) {
-      sp[threadIdx.x] = make_dvec4(pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], mass[j]);
-      sl[threadIdx.x] = make_dvec4(lam[3 * j], lam[3 * j + 1], lam[3 * j + 2], 0.0);
-    }
-    __syncthreads();
-    const int jn = (j1 - c) < AJ_THREADS ? (int)(j1 - c) : AJ_THREADS;
-    for (int t = 0; t < jn; t++) {
-      if (c + t == k) continue;
-      const dvec4 P = sp[t], L = sl[t];
-      const double dx = P.x - xk, dy = P.y - yk, dz = P.z - zk;
-      const double s = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-      double r2, q;  // s^-1 and s^(-3/2) on the integer pipes; FP64 Newton steps outside its range
-      if (!emu::rsqrt_powers(s, r2, q)) {
-        const double r = rsqrt_nr(s);
-        r2 = r * r;
-        q = r2 * r;
+    if (j < n) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        src[k][tid] = pos[3 * j + k];
+        src[4 + k][tid] = lam[3 * j + k];
       }
-      const double p = 3.0 * q * r2;
-      const double ux = mk * L.x - P.w * lxk, uy = mk * L.y - P.w * lyk, uz = mk * L.z - P.w * lzk;
-      const double du = fma(dx, ux, fma(dy, uy, dz * uz));
-      const double pd = p * du;
-      gx = fma(q, ux, fma(-pd, dx, gx));
-      gy = fma(q, uy, fma(-pd, dy, gy));
-      gz = fma(q, uz, fma(-pd, dz, gz));
-      gm = fma(-q, fma(L.x, dx, fma(L.y, dy, L.z * dz)), gm);
+      src[3][tid] = mass[j];
+    }
+#pragma unroll
+    for (int w = 0; w < NW; w++)
+#pragma unroll
+      for (int c = 0; c < 4; c++) col[w][c][tid] = 0.0;
+    __syncthreads();
+    const int jn = i < n ? (int)(n - j0 < AJ_THREADS ? n - j0 : AJ_THREADS) : 0;  // sources to take
+    for (int k = d | k0 ? k0 : 1; k < k1; k++) {  // k = 0 of the block with itself: the particle itself
+      const int q = (tid + k) & (AJ_THREADS - 1);
+      if (q < jn) {
+        const double dx = src[0][q] - xi, dy = src[1][q] - yi, dz = src[2][q] - zi;
+        const double s = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
+        double r2, r3;  // s^-1 and s^(-3/2) on the integer pipes; FP64 Newton steps outside its range
+        if (!emu::rsqrt_powers(s, r2, r3)) {
+          const double r = rsqrt_nr(s);
+          r2 = r * r;
+          r3 = r2 * r;
+        }
+        const double p = 3.0 * r3 * r2, mj = src[3][q];
+        const double lx = src[4][q], ly = src[5][q], lz = src[6][q];
+        const double ux = mi * lx - mj * lxi, uy = mi * ly - mj * lyi, uz = mi * lz - mj * lzi;
+        const double du = fma(dx, ux, fma(dy, uy, dz * uz));
+        const double pd = p * du;
+        gx = fma(r3, ux, fma(-pd, dx, gx));
+        gy = fma(r3, uy, fma(-pd, dy, gy));
+        gz = fma(r3, uz, fma(-pd, dz, gz));
+        gm = fma(-r3, fma(lx, dx, fma(ly, dy, lz * dz)), gm);
+        if (d) {
+          double* c = &col[warp][0][q];
+          c[0] = fma(-r3, ux, fma(pd, dx, c[0]));
+          c[AJ_THREADS] = fma(-r3, uy, fma(pd, dy, c[AJ_THREADS]));
+          c[2 * AJ_THREADS] = fma(-r3, uz, fma(pd, dz, c[2 * AJ_THREADS]));
+          c[3 * AJ_THREADS] = fma(r3, fma(lxi, dx, fma(lyi, dy, lzi * dz)), c[3 * AJ_THREADS]);
+        }
+      }
+      __syncwarp();  // the neighbouring lane takes this source next
+    }
+    __syncthreads();
+    if (d) {
+      double* o = part_j + ((int64_t)blockIdx.y * dmax * parts + e - parts) * 4 * AJ_THREADS + tid;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        double a = col[0][c][tid];
+#pragma unroll
+        for (int w = 1; w < NW; w++) a += col[w][c][tid];
+        o[c * AJ_THREADS] = a;
+      }
     }
   }
-  if (valid) {
-    double* o = part + (split * n + k) * 4;
-    o[0] = gx;
-    o[1] = gy;
-    o[2] = gz;
-    o[3] = gm;
-  }
+  double* o = part_i + ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 4 * AJ_THREADS + tid;
+  o[0] = gx;
+  o[AJ_THREADS] = gy;
+  o[2 * AJ_THREADS] = gz;
+  o[3 * AJ_THREADS] = gm;
 }
 
 // ---------------------------------------------------------------------------
@@ -260,19 +299,6 @@ __global__ void __launch_bounds__(VJ_THREADS, 4)
   }
 }
 
-__global__ void vjp_reduce_f64_kernel(const double* __restrict__ part, int splits, int64_t n,
-                                      double* __restrict__ gpos, double* __restrict__ gmass) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  double a[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int s = 0; s < splits; s++)
-    for (int q = 0; q < 4; q++) a[q] += part[((int64_t)s * n + k) * 4 + q];
-  gpos[3 * k] = a[0];
-  gpos[3 * k + 1] = a[1];
-  gpos[3 * k + 2] = a[2];
-  if (gmass) gmass[k] = a[3];
-}
-
 // One thread per target and component: (hi, lo) pairs are 8 bytes of consecutive threads,
 // and the splits' sums are added in split order (one thread per target with 4-byte loads 32
 // bytes apart took 41 us at N = 16,384, 32 splits).
@@ -417,22 +443,27 @@ __global__ void __launch_bounds__(AJ_THREADS)
 }
 
 // Adds the sums of rows row0 .. row0 + rows - 1: a particle's own row, split by split, then
-// the rows that met its block as a column, in row order.
-__global__ void potential_reduce_kernel(const double* __restrict__ part_i, const double* __restrict__ part_j, int64_t n,
-                                        int nblocks, int row0, int rows, int splits, double* __restrict__ phi) {
+// the rows that met its block as a column, in row order.  C sums per particle, one per
+// blockIdx.y: the first of them to out (stride C < 4 ? C : 3), a fourth to out4.
+template <int C>
+__global__ void pairs_reduce_kernel(const double* __restrict__ part_i, const double* __restrict__ part_j, int64_t n,
+                                    int nblocks, int row0, int rows, int parts, int splits,
+                                    double* __restrict__ out, double* __restrict__ out4) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const int J = (int)(k / AJ_THREADS), o = (int)(k - (int64_t)J * AJ_THREADS), dmax = nblocks / 2;
-  double a = row0 ? phi[k] : 0.0;
+  const int c = blockIdx.y;
+  double* to = c == 3 ? out4 + k : out + k * (C < 4 ? C : 3) + c;
+  const int J = (int)(k / AJ_THREADS), o = (int)(k - (int64_t)J * AJ_THREADS) + c * AJ_THREADS, dmax = nblocks / 2;
+  double a = row0 ? *to : 0.0;
   if (J >= row0 && J < row0 + rows)
-    for (int s = 0; s < splits; s++) a += part_i[((int64_t)(J - row0) * splits + s) * AJ_THREADS + o];
+    for (int s = 0; s < splits; s++) a += part_i[((int64_t)(J - row0) * splits + s) * C * AJ_THREADS + o];
   for (int r = 0; r < rows; r++) {
     const int I = row0 + r;
     const int d = J >= I ? J - I : J - I + nblocks;
     if (d < 1 || d > dmax || (2 * d == nblocks && I >= nblocks / 2)) continue;
-    a += part_j[((int64_t)r * dmax + d - 1) * AJ_THREADS + o];
+    for (int p = 0; p < parts; p++) a += part_j[(((int64_t)r * dmax + d - 1) * parts + p) * C * AJ_THREADS + o];
   }
-  phi[k] = a;
+  *to = a;
 }
 
 // Mass-weighted centre for the FP32 sources, in 256 chains (particles t, t + 256, ...) of
@@ -525,14 +556,37 @@ struct AdjWS {
 static AdjWS g_adj[64];
 static std::mutex g_adj_mu;
 
-// Number of source splits so that the grid fills the GPU about twice over.
-static int64_t choose_splits(int64_t n, int num_sms) {
-  const int64_t tiles = (n + AJ_THREADS - 1) / AJ_THREADS;
-  int64_t want = (4LL * num_sms * 4 + tiles - 1) / tiles;  // ~4 CTAs of 128 threads per SM, x4
-  const int64_t max_splits = (n + AJ_THREADS - 1) / AJ_THREADS;
-  if (want > max_splits) want = max_splits;
-  if (want < 1) want = 1;
-  return want;
+constexpr size_t PAIR_SCRATCH = 256u << 20;  // bytes of column sums held at once, at most
+
+// How an unordered-pair sum of `comps` values per particle is laid out.
+struct PairPlan {
+  int nblocks, parts, len;  // CTAs' shares of a pair of blocks, and how many of them one CTA takes
+  int64_t rows, splits;     // rows of one launch, CTAs per row
+};
+
+static int plan_pairs(AdjWS& ws, int64_t n, int comps, int parts, int num_sms, PairPlan* out) {
+  const int nblocks = (int)((n + AJ_THREADS - 1) / AJ_THREADS), dmax = nblocks / 2;
+  const size_t row_bytes = (size_t)(dmax > 0 ? dmax : 1) * parts * comps * AJ_THREADS * sizeof(double);
+  // the rows of one launch: all that the scratch holds, fewer when memory is short
+  int64_t rows = (int64_t)(PAIR_SCRATCH / row_bytes);
+  if (rows > nblocks) rows = nblocks;
+  if (rows < 1) rows = 1;
+  for (;;) {
+    int64_t splits = (64LL * num_sms + rows - 1) / rows;  // eight waves of about eight CTAs per SM
+    const int64_t most = (int64_t)(dmax + 1) * parts;
+    if (splits > most) splits = most;
+    out->len = (int)((most + splits - 1) / splits);
+    splits = (most + out->len - 1) / out->len;
+    int rc = ensure(ws.part, (size_t)rows * splits * comps * AJ_THREADS * sizeof(double));
+    if (rc == GH_OK) rc = ensure(ws.part_j, (size_t)rows * row_bytes);
+    out->nblocks = nblocks;
+    out->parts = parts;
+    out->rows = rows;
+    out->splits = splits;
+    if (rc != GH_ERR_OOM || rows == 1) return rc;
+    clear_error();
+    rows = (rows + 7) / 8;
+  }
 }
 
 int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, const double* lam, int precision,
@@ -547,18 +601,28 @@ int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, con
   DeviceInfo di;
   GH_TRY(device_info(&di));
   AdjWS& ws = g_adj[di.device];
-  const int64_t splits = choose_splits(n, di.num_sms);
-  const int64_t jlen = (n + splits - 1) / splits;
-  const dim3 grid((unsigned)((n + AJ_THREADS - 1) / AJ_THREADS), (unsigned)splits);
   const unsigned rb = (unsigned)((n + 255) / 256);
   if (precision == GH_PREC_FP64) {
-    GH_TRY(ensure(ws.part, (size_t)splits * n * 4 * sizeof(double)));
-    prof_begin(st);
-    vjp_f64_kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, lam, n, eps * eps, jlen, (double*)ws.part.ptr);
-    prof_end(st);
-    GH_LAUNCH_CHECK();
-    vjp_reduce_f64_kernel<<<rb, 256, 0, st>>>((const double*)ws.part.ptr, (int)splits, n, gpos, gmass);
-    GH_LAUNCH_CHECK();
+    PairPlan pp;
+    // A pair of blocks is a chain of 128 pairs per lane, some 200 us; shares of it where the
+    // pairs of blocks are few: N = 100 32 shares 167 -> 15 us, 1000 8 shares 227 -> 76, 6000
+    // 1329 -> 1277; more blocks lose (16,384 8981 -> 9220).
+    const int64_t nb = (n + AJ_THREADS - 1) / AJ_THREADS, meets = nb * (nb / 2 + 1);
+    const int parts = meets < 8 ? 32 : (meets < 1200 ? 8 : 1);
+    GH_TRY(plan_pairs(ws, n, 4, parts, di.num_sms, &pp));
+    for (int row0 = 0; row0 < pp.nblocks; row0 += (int)pp.rows) {
+      const int here = pp.nblocks - row0 < pp.rows ? pp.nblocks - row0 : (int)pp.rows;
+      prof_begin(st);
+      vjp_pairs_f64_kernel<<<dim3((unsigned)pp.splits, (unsigned)here), AJ_THREADS, 0, st>>>(
+          pos, mass, lam, n, eps * eps, pp.nblocks, row0, pp.parts, pp.len, (double*)ws.part.ptr,
+          (double*)ws.part_j.ptr);
+      prof_end(st);
+      GH_LAUNCH_CHECK();
+      pairs_reduce_kernel<4><<<dim3(rb, gmass ? 4 : 3), 256, 0, st>>>(
+          (const double*)ws.part.ptr, (const double*)ws.part_j.ptr, n, pp.nblocks, row0, here, pp.parts, (int)pp.splits, gpos,
+          gmass);
+      GH_LAUNCH_CHECK();
+    }
     return GH_OK;
   }
   GH_TRY(ensure(ws.src, (size_t)n * sizeof(float4)));
@@ -766,8 +830,6 @@ int dkd_backward_chain(const double* cx, const double* cv, const int64_t* seg, i
   return GH_OK;
 }
 
-constexpr size_t POT_SCRATCH = 256u << 20;  // bytes of column sums held at once, at most
-
 int potential(const double* pos, const double* mass, int64_t n, double eps, double* phi, cudaStream_t st) {
   if (n < 0) return set_error(GH_ERR_ARG, "negative particle count");
   if (!(eps >= 0.0)) return set_error(GH_ERR_ARG, "eps must be >= 0 (got %g)", eps);
@@ -777,40 +839,23 @@ int potential(const double* pos, const double* mass, int64_t n, double eps, doub
   DeviceInfo di;
   GH_TRY(device_info(&di));
   AdjWS& ws = g_adj[di.device];
-  const int nblocks = (int)((n + AJ_THREADS - 1) / AJ_THREADS), dmax = nblocks / 2;
-  const size_t row_bytes = (size_t)(dmax > 0 ? dmax : 1) * AJ_THREADS * sizeof(double);
-  // the rows of one launch: all that the scratch holds, fewer when memory is short
-  int64_t rows = (int64_t)(POT_SCRATCH / row_bytes);
-  if (rows > nblocks) rows = nblocks;
-  if (rows < 1) rows = 1;
-  int64_t splits = 1;
-  int dlen = 1;
-  for (;;) {
-    splits = (64LL * di.num_sms + rows - 1) / rows;  // eight waves of about eight CTAs per SM
-    if (splits > dmax + 1) splits = dmax + 1;
-    dlen = (int)((dmax + 1 + splits - 1) / splits);
-    splits = (dmax + 1 + dlen - 1) / dlen;
-    int rc = ensure(ws.part, (size_t)rows * splits * AJ_THREADS * sizeof(double));
-    if (rc == GH_OK) rc = ensure(ws.part_j, (size_t)rows * row_bytes);
-    if (rc == GH_OK) break;
-    if (rc != GH_ERR_OOM || rows == 1) return rc;
-    clear_error();
-    rows = (rows + 7) / 8;
-  }
+  PairPlan pp;
+  GH_TRY(plan_pairs(ws, n, 1, 1, di.num_sms, &pp));
   GH_TRY(ensure(ws.origin, sizeof(unsigned long long)));
   unsigned long long* largest = (unsigned long long*)ws.origin.ptr;
   GH_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(*largest), st));
   const int64_t need = (3 * n + 255) / 256, cap = 2LL * di.num_sms;
   largest_coordinate_kernel<<<(unsigned)(need < cap ? need : cap), 256, 0, st>>>(pos, 3 * n, largest);
   GH_LAUNCH_CHECK();
-  for (int row0 = 0; row0 < nblocks; row0 += (int)rows) {
-    const int here = nblocks - row0 < rows ? nblocks - row0 : (int)rows;
-    const dim3 grid((unsigned)splits, (unsigned)here);
-    potential_pairs_kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, n, eps * eps, largest, nblocks, row0, dlen,
+  for (int row0 = 0; row0 < pp.nblocks; row0 += (int)pp.rows) {
+    const int here = pp.nblocks - row0 < pp.rows ? pp.nblocks - row0 : (int)pp.rows;
+    const dim3 grid((unsigned)pp.splits, (unsigned)here);
+    potential_pairs_kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, n, eps * eps, largest, pp.nblocks, row0, pp.len,
                                                         (double*)ws.part.ptr, (double*)ws.part_j.ptr);
     GH_LAUNCH_CHECK();
-    potential_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-        (const double*)ws.part.ptr, (const double*)ws.part_j.ptr, n, nblocks, row0, here, (int)splits, phi);
+    pairs_reduce_kernel<1><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const double*)ws.part.ptr,
+                                                                       (const double*)ws.part_j.ptr, n, pp.nblocks,
+                                                                       row0, here, 1, (int)pp.splits, phi, nullptr);
     GH_LAUNCH_CHECK();
   }
   return GH_OK;
