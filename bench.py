@@ -466,9 +466,9 @@ def measure_energy_drift(dev, n=262144, steps=10):
 
 def measure_tree(dev, n=1 << 20, steps=2, fp64_peak=None):
     """Config 2: Hernquist + exponential disk, particle-steps/s of DKD steps with the tree.
-    For the FP64 walk also its FP64-pipe fraction: 10 FP64-pipe operations per
-    interaction (3 differences, 3 FMAs for r^2, one product, 3 accumulating FMAs) over
-    the timed walk, against the FP64 peak measured in the same process."""
+    For the FP64 walk also its FP64-pipe fraction: 6 FP64-pipe operations per interaction
+    (3 differences, 3 accumulating FMAs; the factor is fixed point on the integer pipes)
+    over the timed walk, against the FP64 peak measured in the same process."""
     import numpy as np
     import torch
 
@@ -516,7 +516,7 @@ def measure_tree(dev, n=1 << 20, steps=2, fp64_peak=None):
                               "record_read_frac_of_measured_l2": rec_bytes / walk_s / l2,
                               "per_target_record_gbs": 48 * c["target_visits"] / walk_s / 1e9}
             if prec == "fp64" and fp64_peak:
-                out[key][prec]["fp64_pipe_frac"] = 10.0 * c["interactions"] / walk_s / fp64_peak
+                out[key][prec]["fp64_pipe_frac"] = 6.0 * c["interactions"] / walk_s / fp64_peak
     # CPU reference tree (the oracle restatement of _jbgrav.c) on a sample of targets:
     # its serial build plus the threaded walk of 16384 targets scaled to all N targets
     # (the faster of two calls).

@@ -23,6 +23,7 @@
 //      192-bit fixed-point prefix sums, rounded to FP64 once (the reference rounds
 //      after every particle it adds, in insertion order, so the last bits of an
 //      internal COM can differ), and the centre of mass is first moment over mass.
+// Small systems take the same steps in six launches, the keys ranked by comparison.
 // Walk: one warp per 32 consecutive targets in key order.  Each lane applies the
 // reference's test "leaf or size/|center - x| < theta" (_jbgrav.c:496-502) to every
 // cell its own traversal reaches; the warp visits the union of those cells in
@@ -30,7 +31,8 @@
 // from hi/lo split coordinates with a 1e-4 relative margin; inside the margin it is
 // recomputed with the reference's FP64 operations, so every lane takes exactly the
 // reference's decisions.  Accepted cells contribute (COM - x) m / (r^2 + eps^2)^1.5 in
-// FP64, with the reference's zero for r^2 + eps^2 == 0 (_jbgrav.c:514-520).
+// FP64, with the reference's zero for r^2 + eps^2 == 0 (_jbgrav.c:514-520).  An FP64 walk
+// of few targets is split over several warps per 32 of them by ranges of the preorder.
 #include <cmath>
 #include <mutex>
 
@@ -978,7 +980,7 @@ __global__ void __launch_bounds__(SC_CELL_THREADS)
 // Walk
 // ---------------------------------------------------------------------------
 constexpr int TW_THREADS = 128;
-constexpr int TW_MINB = 9;  // 56 registers, no spills: 36 warps per SM (measured fastest)
+constexpr int TW_MINB = 9;  // 56 registers: 36 warps per SM (10: 48 registers, spills, slower)
 
 __device__ __forceinline__ double rsqrt_f64(double s) {
   double y;
