@@ -40,7 +40,7 @@ __device__ __forceinline__ double rsqrt_nr(double s) {
 // (cyclic; of two opposite blocks only the lower row takes the pairs), a warp's lanes at
 // different sources of a block, whose sums wait in shared memory, one set per warp.  Where that is few
 // CTAs, `parts` of them share a pair of blocks.
-// FP64-pipe bound: 38 operations per unordered pair against 2 x 28 with ordered ones (per
+// FP64-pipe bound (93 % busy at N = 16,384): 38 operations per unordered pair against 2 x 28 with ordered ones (per
 // VJP, N = 500 160 -> 39 us, 2000 253 -> 184, 4096 877 -> 625, 16,384 13.08 -> 8.97 ms).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(AJ_THREADS)
