@@ -1127,15 +1127,15 @@ __device__ __forceinline__ bool walk_is_chain(const WalkRec* __restrict__ nR, in
 }
 
 // Mixed walk.  A step is a chain (record, opening test, the lanes' next node) of some 50
-// instructions, most of them waiting for the one before.  So a step has one branch, for the rare exact test, its interaction is formed by every lane, the fold
-// is a loop of its own around the steps, and the position for the exact test is read again
-// instead of held.  (N = 262,144: 50 -> 48 instructions a step, but 62 -> 70 %
-// of the issue slots, waits on the pipes 3.2 -> 2.2 warps per issue.)  N = 16,384 theta 0.7
-// 408 -> 318 us, 60,013 505 -> 399, 1,048,576 theta
-// 0.5 9.62 -> 8.49 ms (the FP64 walk, whose steps also end in rounds of interactions: 344 ->
-// 322 us, 1141 -> 1085, 17.34 -> 17.20 ms at theta 0.7).  More warps with fewer registers
-// (spills), the next record's load ahead of the interaction, and votes in place of the
-// minimum were all slower.
+// instructions, most of them waiting for the one before.  So a step has one branch, for the
+// rare exact test, its interaction is formed by every lane, the fold is a loop of its own
+// around the steps, and the position for the exact test is read again instead of held.
+// (N = 262,144: 50 -> 48 instructions a step, but 62 -> 70 % of the issue slots, waits on
+// the pipes 3.2 -> 2.2 warps per issue.)  N = 16,384 theta 0.7 408 -> 318 us, 60,013 505 ->
+// 399, 1,048,576 theta 0.5 9.62 -> 8.49 ms (the FP64 walk, whose steps also end in rounds of
+// interactions: 344 -> 322 us, 1141 -> 1085, 17.34 -> 17.20 ms at theta 0.7).  More warps
+// with fewer registers (spills), the next record's load ahead of the interaction, and votes
+// in place of the minimum were all slower.
 template <bool GUARD, bool STATS, class Epi>
 __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
     tree_walk_kernel(const WalkRec* __restrict__ nR, const dvec4* __restrict__ nC, const int* __restrict__ nodes,
