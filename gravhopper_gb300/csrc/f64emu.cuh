@@ -471,8 +471,9 @@ GH_EMU_HD bool aligned_norm2(double dx, double dy, double dz, int Ee, uint64_t W
 
 // Seed of 1/sqrt(n), n = N10 2^-62, as Y0 = y0 2^30 in (2^29, 2^30], and the residual
 // h = 1 - n y0^2 as H = h 2^60.  The approximation (relative error at most 2^-22.9), the
-// conversion of n and the seed's 23 bits leave |h| < 2^-20; host builds, whose seed may be
-// any, check it.
+// conversion of n and the seed's 23 bits leave |h| < 2^-20.  The device does not check that,
+// so n has to lie in [1, 4); host builds, whose seed may be any, do, unless GH_EMU_DEVICE_SEED
+// is defined (tests).
 GH_EMU_HD bool rsqrt_seed_residual(uint64_t N10, uint32_t& Y0, uint64_t& Y0sq, int64_t& H) {
   const uint32_t hi = (uint32_t)(N10 >> 32);
 #ifdef __CUDA_ARCH__
@@ -484,7 +485,7 @@ GH_EMU_HD bool rsqrt_seed_residual(uint64_t N10, uint32_t& Y0, uint64_t& Y0sq, i
 #endif
   Y0sq = (uint64_t)Y0 * Y0;  // y0^2 2^60, at most a little above 2^60
   H = (int64_t)((1ull << 60) - umulhi_low(N10, Y0sq << 2));
-#ifdef __CUDA_ARCH__
+#if defined(__CUDA_ARCH__) || defined(GH_EMU_DEVICE_SEED)
   return true;
 #else
   return (uint64_t)(H + (1ll << 40)) < (1ull << 41);
@@ -588,7 +589,7 @@ GH_EMU_HD int clz32(uint32_t v) {
 // inv_distance of two fixed-point positions, without a floating-point difference.  e_eps
 // and W as align_eps2 gives them (e_eps = Ee - 1023), room = E - e_eps >= 0 (a large number
 // for eps = 0): the squares are aligned at the largest difference's leading bit, or at the
-// softening's.  False when both lie below 2^(E - 32).
+// softening's.  False below sqrt(d^2 + eps^2) = 2^(E - 31), where n would leave [1, 4).
 GH_EMU_HD bool inv_distance_fix96(const Fix96* a, const Fix96* b, int E, int room, uint64_t W, double& out) {
   uint32_t x0, x1, x2, y0, y1, y2, z0, z1, z2;
   fix96_distance(a[0], b[0], x0, x1, x2);
@@ -601,7 +602,7 @@ GH_EMU_HD bool inv_distance_fix96(const Fix96* a, const Fix96* b, int E, int roo
   const uint64_t Z = ((uint64_t)shl_funnel(z1, z2, sh) << 32) | shl_funnel(z0, z1, sh);
   const uint64_t S = square_hi(X) + square_hi(Y) + square_hi(Z) + shr_clamp(W, 2 * (room - sh));
   const int big = (S >> 62) != 0;
-  return ((S >> 59) != 0) & inv_root_rn(big ? S : S << 2, E - sh + big, out);
+  return ((S >> 60) != 0) & inv_root_rn(big ? S : S << 2, E - sh + big, out);
 }
 
 GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
