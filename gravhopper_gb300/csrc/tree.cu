@@ -1852,6 +1852,7 @@ int tree_force(const double* pos, const double* mass, int64_t np, const double* 
   const bool self = (tpos == nullptr);
   if (self) nt = np;
   if (nt == 0) return GH_OK;
+  if (!acc || (np > 0 && (!pos || !mass))) return set_error(GH_ERR_ARG, "null buffer passed to tree force");
   if (np == 0) {
     GH_CUDA_TRY(cudaMemsetAsync(acc, 0, (size_t)nt * 3 * sizeof(double), st));
     return GH_OK;
