@@ -631,5 +631,17 @@ GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, 
   return true;
 }
 
+// m s^(-3/2) = m of a zero mass, where mass_inv_cube refuses nothing but that: false for
+// another mass or outside the range of aligned_norm2 (there the power may overflow).
+GH_EMU_HD bool zero_mass_inv_cube(double m, double dx, double dy, double dz, int Ee, double& out) {
+  const int Ex = (int)(dbits(dx) >> 52) & 0x7FF, Ey = (int)(dbits(dy) >> 52) & 0x7FF, Ez = (int)(dbits(dz) >> 52) & 0x7FF;
+  int E = Ex > Ey ? Ex : Ey;
+  E = Ez > E ? Ez : E;
+  E = Ee > E ? Ee : E;
+  if ((dbits(m) << 1) != 0 || (unsigned)(E - 873) > 300u) return false;
+  out = m;
+  return true;
+}
+
 }  // namespace emu
 }  // namespace gh
