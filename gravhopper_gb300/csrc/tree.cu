@@ -806,6 +806,10 @@ __global__ void __launch_bounds__(MS_THREADS) moments_tiles_kernel(FxMoments* __
 constexpr int SB_MAX = 8192;
 constexpr int SB_ITEMS = SB_MAX / SB_THREADS;
 enum SmallStatus { SB_OK = 0, SB_BAD = 1, SB_TIE = 2, SB_ROOM = 3 };
+// A tie usually recurs in the next step of the same system, and then the small build and the
+// walk queued on it were for nothing, so its particle count keeps to the general build until
+// as many builds of it in a row had no tie (several systems of one count may take turns).
+constexpr int SB_TIE_BUILDS = 4;
 
 // Rank of each key among all (words and index), 16 particles x 16 slices of the others per
 // block; writes the keys and indices in order.
@@ -1437,7 +1441,9 @@ struct TreeWS {
   Buffer cells;               // (internal cell, opener) pairs
   int* host_flags = nullptr;  // pinned: the 8 device flags, nnodes, the root's non-finite flag; [10..11] small build
   cudaEvent_t small_built = nullptr;
-  int64_t small_tie_n = -1;   // particle count of the last small build whose two-word keys tied
+  // Per particle count: how many more general builds, from the last whose two-word keys tied
+  // on, before the small build is tried again.
+  uint8_t small_tied[SB_MAX + 1] = {};
   int64_t small_room = 0;     // nodes that a small build may write
   int words = TREE_MIN_WORDS;
   int64_t full_sort_n = -1;  // particle count whose last build needed the full multi-word sort
@@ -1531,7 +1537,7 @@ static int small_finish(TreeWS& ws, BuiltTree* bt, bool* again) {
   switch (status[0]) {
     case SB_OK: return GH_OK;
     case SB_BAD: return bad_input();
-    case SB_TIE: ws.small_tie_n = bt->n; break;
+    case SB_TIE: ws.small_tied[bt->n] = SB_TIE_BUILDS; break;
     default: ws.small_room = (int64_t)status[1] + status[1] / 4;
   }
   *again = true;
@@ -1552,7 +1558,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
   if (n > (1LL << 24)) return set_error(GH_ERR_ARG, "tree: at most 16777216 particles (got %lld)", (long long)n);
   if (!ws.host_flags) GH_CUDA_TRY(cudaMallocHost((void**)&ws.host_flags, 16 * sizeof(int)));
   const bool wait_fault = inject_take(GH_INJECT_TREE_WAIT);  // test hook: as if a look-back wait had run out
-  if (n <= SB_MAX && n != ws.small_tie_n && !sort_targets && !wait_fault) {
+  if (n <= SB_MAX && !ws.small_tied[n] && !sort_targets && !wait_fault) {
     GH_TRY(small_build(ws, pos, mass, n, eps, st, out));
     if (defer) return GH_OK;
     bool again;
@@ -1661,6 +1667,13 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
   const int words = ws.words;
   const int maxdepth = ws.host_flags[1];
   const int nnodes = ws.host_flags[8];
+  if (n <= SB_MAX) {
+    uint8_t& tied = ws.small_tied[n];
+    if (maxdepth > 2 * KEY_LEVELS)  // a leaf below both words' levels: they tied
+      tied = SB_TIE_BUILDS;
+    else if (tied)
+      tied--;
+  }
   // 4. nodes
   GH_TRY(ensure(ws.nA, (size_t)nnodes * sizeof(WalkRec)));
   GH_TRY(ensure(ws.nC, (size_t)nnodes * sizeof(dvec4)));
