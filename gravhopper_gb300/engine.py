@@ -20,15 +20,12 @@ def _check(t, name, shape_tail=None):
         raise ValueError(f"{name} must have shape (N,{shape_tail})")
 
 
-def _check_len(t, name, n):
-    if t.shape[0] != n:
-        raise ValueError(f"{name} and pos have different lengths")
-
-
 def _points(force_pos, pos):
     """Address of the target points; the library takes a null one, as an empty tensor's is,
     to ask for the self-force, so any other stands in for that."""
-    return _capi.ptr(pos if force_pos is not None and force_pos.shape[0] == 0 else force_pos)
+    if force_pos is None:
+        return None
+    return force_pos.data_ptr() or pos.data_ptr()
 
 
 def _check_room(t, name, count):
@@ -49,7 +46,8 @@ def direct_force(pos, mass, eps, force_pos=None, precision="fp64", out=None, str
     n_out = pos.shape[0] if force_pos is None else force_pos.shape[0]
     if out is None:
         out = torch.empty((n_out, 3), dtype=torch.float64, device=pos.device)
-    _check_room(out, "out", 3 * n_out)
+    else:
+        _check_room(out, "out", 3 * n_out)
     _capi.call("gh_direct_dev", _capi.ptr(pos), _capi.ptr(mass), pos.shape[0], _points(force_pos, pos),
                0 if force_pos is None else force_pos.shape[0], float(eps),
                _capi.PRECISIONS[precision], _capi.ptr(out), _capi.stream_handle(stream))
@@ -69,7 +67,8 @@ def tree_force(pos, mass, eps, theta=0.7, force_pos=None, out=None, stream=None,
     n_out = pos.shape[0] if force_pos is None else force_pos.shape[0]
     if out is None:
         out = torch.empty((n_out, 3), dtype=torch.float64, device=pos.device)
-    _check_room(out, "out", 3 * n_out)
+    else:
+        _check_room(out, "out", 3 * n_out)
     _capi.call("gh_tree_dev", _capi.ptr(pos), _capi.ptr(mass), pos.shape[0], _points(force_pos, pos),
                0 if force_pos is None else force_pos.shape[0], float(eps), float(theta),
                _capi.PRECISIONS[precision], _capi.ptr(out), _capi.stream_handle(stream))
@@ -147,14 +146,16 @@ def direct_vjp(pos, mass, eps, cot, precision="fp64", grad_pos=None, grad_mass=N
     _check(mass, "mass")
     _check(cot, "cot", 3)
     n = pos.shape[0]
-    _check_len(mass, "mass", n)
-    _check_len(cot, "cot", n)
+    if mass.shape[0] != n or cot.shape[0] != n:
+        raise ValueError("pos, mass and cot have different lengths")
     if grad_pos is None:
         grad_pos = torch.empty((n, 3), dtype=torch.float64, device=pos.device)
+    else:
+        _check_room(grad_pos, "grad_pos", 3 * n)
     if grad_mass is None:
         grad_mass = torch.empty(n, dtype=torch.float64, device=pos.device)
-    _check_room(grad_pos, "grad_pos", 3 * n)
-    _check_room(grad_mass, "grad_mass", n)
+    else:
+        _check_room(grad_mass, "grad_mass", n)
     _capi.call("gh_direct_vjp_dev", _capi.ptr(pos), _capi.ptr(mass), n, float(eps), _capi.ptr(cot),
                _capi.PRECISIONS[precision], _capi.ptr(grad_pos), _capi.ptr(grad_mass), _capi.stream_handle(stream))
     return grad_pos, grad_mass
@@ -165,10 +166,12 @@ def potential(pos, mass, eps, out=None, stream=None):
     _check(pos, "pos", 3)
     _check(mass, "mass")
     n = pos.shape[0]
-    _check_len(mass, "mass", n)
+    if mass.shape[0] != n:
+        raise ValueError("mass and pos have different lengths")
     if out is None:
         out = torch.empty(n, dtype=torch.float64, device=pos.device)
-    _check_room(out, "out", n)
+    else:
+        _check_room(out, "out", n)
     _capi.call("gh_potential_dev", _capi.ptr(pos), _capi.ptr(mass), n, float(eps), _capi.ptr(out),
                _capi.stream_handle(stream))
     return out
