@@ -146,8 +146,8 @@ def direct_vjp(pos, mass, eps, cot, precision="fp64", grad_pos=None, grad_mass=N
     _check(mass, "mass")
     _check(cot, "cot", 3)
     n = pos.shape[0]
-    if mass.shape[0] != n or cot.shape[0] != n:
-        raise ValueError("pos, mass and cot have different lengths")
+    if mass.numel() < n or cot.numel() < 3 * n:
+        raise ValueError("mass and cot must hold a value for every particle")
     if grad_pos is None:
         grad_pos = torch.empty((n, 3), dtype=torch.float64, device=pos.device)
     else:
@@ -166,8 +166,8 @@ def potential(pos, mass, eps, out=None, stream=None):
     _check(pos, "pos", 3)
     _check(mass, "mass")
     n = pos.shape[0]
-    if mass.shape[0] != n:
-        raise ValueError("mass and pos have different lengths")
+    if mass.numel() < n:
+        raise ValueError("mass must hold a value for every particle")
     if out is None:
         out = torch.empty(n, dtype=torch.float64, device=pos.device)
     else:
