@@ -336,7 +336,8 @@ __global__ void vjp_reduce_mixed_kernel(const float2* __restrict__ part, int spl
 // cycles of an SM as measured, ALU 71 % busy) with two DFMAs on the FP64 pipe (34 of the
 // cycles).  With FP64 differences it took 94 cycles, and the one-sided sum in FP64 296 (three
 // differences, three DFMAs of the squared distance, a comparison, a DFMA, each twice).
-// N = 65,536: 62.9 -> 20.0 -> 11.7 ms; 8192: 996 -> 364 -> 225 us; 1000: 74 -> 70 -> 56.
+// N = 65,536: 62.9 -> 20.0 -> 11.7 ms; 8192: 996 -> 364 -> 225 us; 1000: 74 -> 70 -> 56 -> 27
+// in shares.
 // Two or four targets per thread: the same from N = 30,000 on, slower below (fewer CTAs).
 // ---------------------------------------------------------------------------
 struct PairEps {
@@ -354,11 +355,12 @@ __device__ __forceinline__ bool pair_inv_distance(double dx, double dy, double d
   return s > 0.0;
 }
 
-// Largest |coordinate|, as the bits of a double (they order like the values).
-__global__ void __launch_bounds__(256)
-    largest_coordinate_kernel(const double* __restrict__ pos, int64_t n3, unsigned long long* __restrict__ out) {
+// Largest |coordinate| of pos[i], i = first, first + step, ... below n3, over a warp, as the
+// bits of a double (they order like the values).
+__device__ __forceinline__ unsigned long long largest_of_warp(const double* __restrict__ pos, int64_t first, int64_t step,
+                                                              int64_t n3) {
   unsigned long long m = 0;
-  for (int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x; k < n3; k += (int64_t)gridDim.x * 256) {
+  for (int64_t k = first; k < n3; k += step) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(pos[k]) & 0x7FFFFFFFFFFFFFFFull;
     m = b > m ? b : m;
   }
@@ -367,25 +369,47 @@ __global__ void __launch_bounds__(256)
     const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
     m = q > m ? q : m;
   }
+  return m;
+}
+
+__global__ void __launch_bounds__(256)
+    largest_coordinate_kernel(const double* __restrict__ pos, int64_t n3, unsigned long long* __restrict__ out) {
+  const unsigned long long m =
+      largest_of_warp(pos, (int64_t)blockIdx.x * 256 + threadIdx.x, (int64_t)gridDim.x * 256, n3);
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
+// WHOLE: each pair of blocks by one CTA (the loop over its 128 steps has fixed bounds: 4 %
+// faster at every large N); else in `parts` shares.
+template <bool WHOLE>
 __global__ void __launch_bounds__(AJ_THREADS)
     potential_pairs_kernel(const double* __restrict__ pos, const double* __restrict__ mass, int64_t n, double eps2,
-                           const unsigned long long* __restrict__ largest, int nblocks, int row0, int dlen,
+                           const unsigned long long* __restrict__ largest, int nblocks, int row0, int shares, int len,
                            double* __restrict__ part_i, double* __restrict__ part_j) {
   constexpr int NW = AJ_THREADS / 32;
   __shared__ uint4 src[3][AJ_THREADS];  // (x, y0), (y1, y2, z0, z1), (z2, -, mass): words of the positions
   __shared__ double col[NW][AJ_THREADS];
   const int tid = threadIdx.x, warp = tid >> 5;
   const int I = row0 + blockIdx.y;
-  const int dmax = nblocks / 2;
-  const int d0 = blockIdx.x * dlen, d1 = d0 + dlen < dmax + 1 ? d0 + dlen : dmax + 1;
+  const int dmax = nblocks / 2, parts = WHOLE ? 1 : shares;
+  const int end = (dmax + 1) * parts, e0 = blockIdx.x * len, e1 = e0 + len < end ? e0 + len : end;
+  unsigned long long top_bits;
+  if (largest) {
+    top_bits = *largest;
+  } else {  // one block of particles: no launches for it
+    __shared__ unsigned long long warp_top[NW];
+    const unsigned long long m = largest_of_warp(pos, tid, AJ_THREADS, 3 * n);
+    if ((tid & 31) == 0) warp_top[warp] = m;
+    __syncthreads();
+    top_bits = warp_top[0];
+#pragma unroll
+    for (int w = 1; w < NW; w++) top_bits = warp_top[w] > top_bits ? warp_top[w] : top_bits;
+  }
   PairEps pe;
   pe.eps2 = eps2;
   pe.ok = emu::align_eps2(eps2, pe.E, pe.W);
   // |x| < 2^E; room: how far the softening's leading bit lies below 2^E
-  const int top = (int)(*largest >> 52), E = top - 1022;
+  const int top = (int)(top_bits >> 52), E = top - 1022;
   const int room = pe.W ? E - (pe.E - 1023) : 1 << 20;
   const bool fix = pe.ok && (unsigned)(top - 873) <= 300u && room >= 0;
   const int64_t i = (int64_t)I * AJ_THREADS + tid;
@@ -394,7 +418,8 @@ __global__ void __launch_bounds__(AJ_THREADS)
 #pragma unroll
   for (int k = 0; k < 3; k++) me[k] = emu::to_fix96(i < n ? pos[3 * i + k] : 0.0, E);
   double phi = 0.0;
-  for (int d = d0; d < d1; d++) {
+  for (int e = e0; e < e1; e++) {
+    const int d = e / parts, k0 = (e - d * parts) * (AJ_THREADS / parts), k1 = k0 + AJ_THREADS / parts;
     if (2 * d == nblocks && d > 0 && I >= nblocks / 2) break;  // the lower rows' pairs
     const int J = I + d < nblocks ? I + d : I + d - nblocks;
     const int64_t j0 = (int64_t)J * AJ_THREADS, j = j0 + tid;
@@ -412,7 +437,7 @@ __global__ void __launch_bounds__(AJ_THREADS)
 #pragma unroll
     for (int w = 0; w < NW; w++) col[w][tid] = 0.0;
     __syncthreads();
-    for (int k = d ? 0 : 1; k < AJ_THREADS; k++) {  // k = 0 of the block with itself: the particle itself
+    for (int k = d | k0 ? k0 : 1; k < (WHOLE ? AJ_THREADS : k1); k++) {  // k = 0 of the block with itself: the particle itself
       const int q = (tid + k) & (AJ_THREADS - 1);
       if (q < jn) {
         const uint4 A = src[0][q], B = src[1][q], C = src[2][q];
@@ -436,7 +461,7 @@ __global__ void __launch_bounds__(AJ_THREADS)
       double a = col[0][tid];
 #pragma unroll
       for (int w = 1; w < NW; w++) a += col[w][tid];
-      part_j[((int64_t)blockIdx.y * dmax + d - 1) * AJ_THREADS + tid] = a;
+      part_j[((int64_t)blockIdx.y * dmax * parts + e - parts) * AJ_THREADS + tid] = a;
     }
   }
   part_i[((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * AJ_THREADS + tid] = phi;
@@ -456,6 +481,7 @@ __global__ void pairs_reduce_kernel(const double* __restrict__ part_i, const dou
   const int J = (int)(k / AJ_THREADS), o = (int)(k - (int64_t)J * AJ_THREADS) + c * AJ_THREADS, dmax = nblocks / 2;
   double a = row0 ? *to : 0.0;
   if (J >= row0 && J < row0 + rows)
+#pragma unroll 8
     for (int s = 0; s < splits; s++) a += part_i[((int64_t)(J - row0) * splits + s) * C * AJ_THREADS + o];
   for (int r = 0; r < rows; r++) {
     const int I = row0 + r;
@@ -589,6 +615,16 @@ static int plan_pairs(AdjWS& ws, int64_t n, int comps, int parts, int num_sms, P
   }
 }
 
+// A pair of blocks is a chain of 128 pairs per lane, some 200 us in the VJP and 45 in the
+// potential; shares of it where the pairs of blocks are few.  VJP: N = 100 32 shares 167 -> 15
+// us, 1000 8 shares 227 -> 76, 6000 1329 -> 1277; more blocks lose (16,384 8981 -> 9220).
+// Potential: N = 30 31 -> 17 us (of one block, which finds its own largest coordinate), 129 50
+// -> 23, 1000 55 -> 27, 3000 74 -> 68; more blocks lose (4000 88 -> 96).
+static int pair_shares(int64_t n, bool vjp) {
+  const int64_t nb = (n + AJ_THREADS - 1) / AJ_THREADS, meets = nb * (nb / 2 + 1);
+  return meets < 8 ? 32 : (meets < (vjp ? 1200 : 320) ? 8 : 1);
+}
+
 int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, const double* lam, int precision,
                double* gpos, double* gmass, cudaStream_t st) {
   if (n < 0) return set_error(GH_ERR_ARG, "negative particle count");
@@ -604,12 +640,7 @@ int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, con
   const unsigned rb = (unsigned)((n + 255) / 256);
   if (precision == GH_PREC_FP64) {
     PairPlan pp;
-    // A pair of blocks is a chain of 128 pairs per lane, some 200 us; shares of it where the
-    // pairs of blocks are few: N = 100 32 shares 167 -> 15 us, 1000 8 shares 227 -> 76, 6000
-    // 1329 -> 1277; more blocks lose (16,384 8981 -> 9220).
-    const int64_t nb = (n + AJ_THREADS - 1) / AJ_THREADS, meets = nb * (nb / 2 + 1);
-    const int parts = meets < 8 ? 32 : (meets < 1200 ? 8 : 1);
-    GH_TRY(plan_pairs(ws, n, 4, parts, di.num_sms, &pp));
+    GH_TRY(plan_pairs(ws, n, 4, pair_shares(n, true), di.num_sms, &pp));
     for (int row0 = 0; row0 < pp.nblocks; row0 += (int)pp.rows) {
       const int here = pp.nblocks - row0 < pp.rows ? pp.nblocks - row0 : (int)pp.rows;
       prof_begin(st);
@@ -840,22 +871,27 @@ int potential(const double* pos, const double* mass, int64_t n, double eps, doub
   GH_TRY(device_info(&di));
   AdjWS& ws = g_adj[di.device];
   PairPlan pp;
-  GH_TRY(plan_pairs(ws, n, 1, 1, di.num_sms, &pp));
-  GH_TRY(ensure(ws.origin, sizeof(unsigned long long)));
-  unsigned long long* largest = (unsigned long long*)ws.origin.ptr;
-  GH_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(*largest), st));
-  const int64_t need = (3 * n + 255) / 256, cap = 2LL * di.num_sms;
-  largest_coordinate_kernel<<<(unsigned)(need < cap ? need : cap), 256, 0, st>>>(pos, 3 * n, largest);
-  GH_LAUNCH_CHECK();
+  GH_TRY(plan_pairs(ws, n, 1, pair_shares(n, false), di.num_sms, &pp));
+  unsigned long long* largest = nullptr;
+  if (pp.nblocks > 1) {
+    GH_TRY(ensure(ws.origin, sizeof(unsigned long long)));
+    largest = (unsigned long long*)ws.origin.ptr;
+    GH_CUDA_TRY(cudaMemsetAsync(largest, 0, sizeof(*largest), st));
+    const int64_t need = (3 * n + 255) / 256, cap = 2LL * di.num_sms;
+    largest_coordinate_kernel<<<(unsigned)(need < cap ? need : cap), 256, 0, st>>>(pos, 3 * n, largest);
+    GH_LAUNCH_CHECK();
+  }
   for (int row0 = 0; row0 < pp.nblocks; row0 += (int)pp.rows) {
     const int here = pp.nblocks - row0 < pp.rows ? pp.nblocks - row0 : (int)pp.rows;
     const dim3 grid((unsigned)pp.splits, (unsigned)here);
-    potential_pairs_kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, n, eps * eps, largest, pp.nblocks, row0, pp.len,
-                                                        (double*)ws.part.ptr, (double*)ws.part_j.ptr);
+    const auto kernel = pp.parts == 1 ? potential_pairs_kernel<true> : potential_pairs_kernel<false>;
+    kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, n, eps * eps, largest, pp.nblocks, row0, pp.parts, pp.len,
+                                        (double*)ws.part.ptr, (double*)ws.part_j.ptr);
     GH_LAUNCH_CHECK();
     pairs_reduce_kernel<1><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const double*)ws.part.ptr,
                                                                        (const double*)ws.part_j.ptr, n, pp.nblocks,
-                                                                       row0, here, 1, (int)pp.splits, phi, nullptr);
+                                                                       row0, here, pp.parts, (int)pp.splits, phi,
+                                                                       nullptr);
     GH_LAUNCH_CHECK();
   }
   return GH_OK;
