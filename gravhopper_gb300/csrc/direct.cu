@@ -3,6 +3,7 @@
 
 #include "direct.cuh"
 #include "engine.h"
+#include "shape_rules.h"
 
 namespace gh {
 
@@ -345,25 +346,6 @@ static int launch_mixed(DirectWS& ws, const float4* src, int64_t np, const float
   prof_end(st);
   GH_LAUNCH_CHECK();
   return GH_OK;
-}
-
-// Targets per CTA of the ordered kernel: the fewest FP64-pipe cycles per source on the SM
-// that holds most CTAs.  A CTA of t targets takes 9 t / 32 warp instructions per source for
-// its pair terms and one, however few of its lanes take part, for its sums.  Force: N = 1500
-// 92 us with 5 against 110 with 4, 2000 153 with 7 against 176 with 4, 4000 496 with 7
-// against 566 with 8; from 6000 on 8 is best (3, 6 and 10 nowhere).
-static int ordered_targets(int64_t nt, int num_sms) {
-  int best = 8;
-  int64_t least = -1;
-  for (const int t : {8, 7, 5, 4, 2}) {
-    const int64_t ctas = (nt + t - 1) / t, per_sm = (ctas + num_sms - 1) / num_sms;
-    const int64_t cost = per_sm * (9 * t + 32);
-    if (least < 0 || cost < least) {
-      least = cost;
-      best = t;
-    }
-  }
-  return best;
 }
 
 template <bool SELF, class Epi>
