@@ -129,9 +129,8 @@ static int g_f64_form = -1;  // -1 by target count, 0 thread per target, 1 order
 // against 443 ms).
 //
 // Few points against many sources, or many against few, leave tiles of 2048 empty or SMs
-// idle: 64 threads x 2 targets with the same chunks of 512 takes 98 us against 240 for 10
-// to 100 points and 100,000 sources, 230 against 277 for 3000 points, 58 against 100 for
-// 50,000 points and 1000 sources; with 5000 sources it is slower (118 against 105).
+// idle: small_tiles (shape_rules.h) says where 64 threads x 2 targets with the same chunks of
+// 512 are faster.
 //
 // An autotuner can replace that table (gh_direct_tune): per epilogue kind (force or
 // fused leapfrog step), rules "from n_min particles on, shape k"; the rule with the
@@ -158,14 +157,14 @@ static int tuned_shape(int64_t n, bool dkd) {
   return best;
 }
 
-static int auto_shape(int64_t np, int64_t nt, bool dkd) {
+static int auto_shape(int64_t np, int64_t nt, bool dkd, int num_sms) {
   const int64_t n = np > nt ? np : nt;
   const int tuned = tuned_shape(n, dkd);
   if (tuned >= 0) return tuned;
   if (n < 12288) return 13;                  // packed, 64 threads, 1 pack, 8 CTAs/SM, chunks of 256
   if (n < 24576) return 14;                  // the same, chunks of 128
   if (dkd && n >= (1 << 17)) return 12;      // scalar, 384 threads x 6 targets
-  if (nt <= 4096 || np <= 2048) return 15;   // packed, 64 threads, 1 pack, 6 CTAs/SM, chunks of 512
+  if (small_tiles(np, nt, num_sms)) return 15;  // packed, 64 threads, 1 pack, 6 CTAs/SM, chunks of 512
   return 10;                                 // scalar, 512 threads x 4 targets
 }
 
@@ -282,7 +281,7 @@ int tune_rule(int64_t n_min, int fused_step, int shape) {
 
 int shape_for(int64_t n, int fused_step) {
   if (g_mixed_shape >= 0) return g_mixed_shape;
-  return auto_shape(n, n, fused_step != 0);
+  return auto_shape(n, n, fused_step != 0, 1);  // no side of it is short: the same for any number of SMs
 }
 
 int set_mixed_shape(int shape) {
@@ -328,7 +327,7 @@ static int launch_mixed(DirectWS& ws, const float4* src, int64_t np, const float
   GH_TRY(device_info(&di));
   const float eps2 = (float)(eps * eps);
   const bool guard = !(eps2 > 0.f);
-  const int shape = g_mixed_shape >= 0 ? g_mixed_shape : auto_shape(np, nt, Epi::kFusedStep);
+  const int shape = g_mixed_shape >= 0 ? g_mixed_shape : auto_shape(np, nt, Epi::kFusedStep, di.num_sms);
   const MixedShape ms = kMixedShapes[shape];
   StreamK sk = mixed_plan(np, nt, mixed_grid_cap(di.num_sms, shape, guard), ms.threads * 2 * ms.packs,
                           ms.jt);

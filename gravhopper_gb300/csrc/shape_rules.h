@@ -34,4 +34,18 @@ inline int ordered_targets(int64_t nt, int num_sms) {
   return best;
 }
 
+// Whether a mixed sum of np sources on nt targets, one side short, takes tiles of 64 threads x
+// 2 targets (six CTAs per SM) instead of 512 x 4 (one): tiles of 2048 targets leave SMs idle
+// or the last wave of them nearly empty, small ones cost a ninth more per pair.  In units of
+// 0.6 us: 120 per unit (tile x chunk of 512 sources) of the busiest CTA with large tiles, 50
+// with small ones, and 1 per CTA that shares a large tile, whose partial sums one CTA adds.
+// Large / small tiles: 100 targets x 100,000 sources 239 / 99 us, 4000 x 300,000 628 / 638,
+// 50,000 targets x 1000 sources 101 / 60, 200,000 x 1500 166 / 192, 1,000,000 x 2048 860 / 924.
+inline bool small_tiles(int64_t np, int64_t nt, int num_sms) {
+  if (nt > 4096 && np > 2048) return false;
+  const int64_t chunks = div_up(np, 512), large = div_up(nt, 2048), small = div_up(nt, 128);
+  const int64_t sharing = div_up(num_sms, large) < chunks ? div_up(num_sms, large) : chunks;
+  return 50 * div_up(small * chunks, 6LL * num_sms) <= 120 * div_up(large * chunks, num_sms) + sharing;
+}
+
 }  // namespace gh
