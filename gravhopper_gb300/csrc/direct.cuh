@@ -226,7 +226,9 @@ __global__ void __launch_bounds__(F64O_THREADS)
                               const double* __restrict__ tpos, int64_t nt, double eps2, Epi epi) {
   static_assert(3 * TB <= 32, "the summing lanes form one warp");
   constexpr int JC = F64O_TERMS / TB;  // sources per chunk
-  constexpr int JP = JC + 1;           // padded rows: the summing lanes hit distinct banks
+  // Padded rows: odd, so that the summing lanes hit distinct banks, but for TB = 5 (90), where
+  // lanes 8 apart share one; 89 is slower there (N = 1520 95.2 us against 93.1).
+  constexpr int JP = JC + 1;
   __shared__ dvec4 src[2][JC];
   __shared__ double term[2][3 * TB][JP];
   __shared__ double tp[TB][3];
