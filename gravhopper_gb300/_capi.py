@@ -29,6 +29,7 @@ GH_ALGO_TREE = 1
 
 GH_INJECT_ALLOC = 1
 GH_INJECT_TREE_WAIT = 2
+GH_INJECT_ALLOC_PASS = 3
 
 PRECISIONS = {"fp64": GH_PREC_FP64, "mixed": GH_PREC_MIXED}
 ALGORITHMS = {"direct": GH_ALGO_DIRECT, "tree": GH_ALGO_TREE}
@@ -219,7 +220,8 @@ def tree_stats_read():
 
 def inject(fault: int, count: int = 1) -> None:
     """Host-side fault injection for tests: the next ``count`` occurrences of ``fault``
-    (GH_INJECT_ALLOC, GH_INJECT_TREE_WAIT) fail as if the device had reported them."""
+    (GH_INJECT_ALLOC, GH_INJECT_TREE_WAIT) fail as if the device had reported them;
+    GH_INJECT_ALLOC_PASS: reservations that pass before GH_INJECT_ALLOC takes effect."""
     call("gh_debug_inject", int(fault), int(count))
 
 

@@ -73,10 +73,10 @@ void prof_end(cudaStream_t st) {
 }
 
 // Pending injected faults, by kind (GH_INJECT_*).
-static std::atomic<long long> g_inject[3];
+static std::atomic<long long> g_inject[4];
 
 bool inject_take(int fault) {
-  if (fault < 1 || fault > 2) return false;
+  if (fault < 1 || fault > 3) return false;
   long long k = g_inject[fault].load(std::memory_order_relaxed);
   while (k > 0)
     if (g_inject[fault].compare_exchange_weak(k, k - 1)) return true;
@@ -84,7 +84,8 @@ bool inject_take(int fault) {
 }
 
 int ensure(Buffer& b, size_t bytes) {
-  if (bytes && inject_take(GH_INJECT_ALLOC)) {
+  if (bytes && g_inject[GH_INJECT_ALLOC].load(std::memory_order_relaxed) > 0 && !inject_take(GH_INJECT_ALLOC_PASS) &&
+      inject_take(GH_INJECT_ALLOC)) {
     // as a growth whose cudaMalloc ran out of memory: the old buffer is gone too
     if (b.ptr) cudaFree(b.ptr);
     b.ptr = nullptr;
@@ -151,7 +152,7 @@ int gh_trace(int enable) {
 
 int gh_debug_inject(int fault, int64_t count) {
   gh::clear_error();
-  if (fault != GH_INJECT_ALLOC && fault != GH_INJECT_TREE_WAIT)
+  if (fault != GH_INJECT_ALLOC && fault != GH_INJECT_TREE_WAIT && fault != GH_INJECT_ALLOC_PASS)
     return gh::set_error(GH_ERR_ARG, "unknown fault kind %d", fault);
   if (count < 0) return gh::set_error(GH_ERR_ARG, "negative fault count");
   gh::g_inject[fault].store(count);

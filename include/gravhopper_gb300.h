@@ -274,12 +274,14 @@ int gh_tree_stats_read(int64_t* out);
 /* Kinds of host-side fault that gh_debug_inject can make the library meet. */
 #define GH_INJECT_ALLOC 1     /* a device workspace allocation runs out of memory */
 #define GH_INJECT_TREE_WAIT 2 /* a tree build finds its radix sort's bounded wait given up */
+#define GH_INJECT_ALLOC_PASS 3 /* reservations that pass before GH_INJECT_ALLOC takes effect */
 
 /* Makes the next `count` occurrences of `fault` fail on the host as if the device had
  * reported them (0 clears it): GH_INJECT_ALLOC fails workspace reservations with
  * GH_ERR_OOM (the reserved buffer is released, as after a failed growth);
- * GH_INJECT_TREE_WAIT makes tree builds return GH_ERR_TIMEOUT after their sort.  Every
- * later call works normally.  For testing the error paths; no GPU fault is involved. */
+ * GH_INJECT_TREE_WAIT makes tree builds return GH_ERR_TIMEOUT after their sort;
+ * GH_INJECT_ALLOC_PASS, with GH_INJECT_ALLOC pending, lets as many reservations pass first,
+ * so that a later one of a call is the one that fails.  Every later call works normally.  For testing the error paths; no GPU fault is involved. */
 int gh_debug_inject(int fault, int64_t count);
 
 /* Runs one pass of the tree build's radix sort over two tiles of keys in which tile 0
