@@ -528,7 +528,8 @@ GH_EMU_HD bool inv_root_rn(uint64_t N10, int e, double& out) {
 GH_EMU_HD bool inv_distance(double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
   uint64_t N10;
   int e;
-  return aligned_norm2(dx, dy, dz, Ee, W, N10, e) & inv_root_rn(N10, e, out);
+  const bool ok = aligned_norm2(dx, dy, dz, Ee, W, N10, e);  // before the root reads N10 and e
+  return inv_root_rn(N10, e, out) & ok;
 }
 
 // Positions in 96-bit two's complement fixed point, unit 2^(E - 94) for |x| < 2^E: exact for
