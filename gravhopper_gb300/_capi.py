@@ -95,6 +95,7 @@ SIGNATURES = {
     "gh_measure_l2_read": (_int, [_vp, _vp]),
     "gh_measure_pair_mix": (_int, [_int, _vp, _vp]),
     "gh_check_inv_cube": (_int, [_i64, _u64, _vp, _vp]),
+    "gh_check_pair_factor": (_int, [_int, _i64, _vp, _vp, _vp]),
     "gh_tree_stats": (_int, [_int]),
     "gh_tree_stats_read": (_int, [_vp]),
     "gh_tree_validate": (_int, [_vp, _vp, _i64, _dbl, _vp, _vp]),
@@ -201,6 +202,17 @@ def check_inv_cube(n: int, seed: int = 1, stream=None):
     out = (ctypes.c_longlong * 2)()
     call("gh_check_inv_cube", int(n), int(seed), ctypes.addressof(out), stream_handle(stream))
     return int(out[0]), int(out[1])
+
+
+def check_pair_factor(kind: int, pairs, stream=None):
+    """Fixed-point pair factors of a device tensor of pairs (gh_check_pair_factor); NaN where
+    refused."""
+    import torch
+    if pairs.dim() != 2 or pairs.shape[1] != (5, 4, 8)[kind] or not pairs.is_contiguous():
+        raise ValueError("pairs must be a contiguous tensor of 5, 4 or 8 values per pair")
+    out = torch.empty(pairs.shape[0], dtype=torch.float64, device=pairs.device)
+    call("gh_check_pair_factor", int(kind), pairs.shape[0], ptr(pairs), ptr(out), stream_handle(stream))
+    return out
 
 
 def tree_stats(enable: bool) -> None:

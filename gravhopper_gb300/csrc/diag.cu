@@ -192,6 +192,36 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The rounded-once pair factors of f64emu.cuh as this device forms them (its own FP32 seed,
+// whose range nothing checks), one per thread: in holds (d, eps^2, m), (d, eps^2) or (a, b,
+// eps^2, box exponent) per pair, out the factor, or NaN where it is refused.
+enum PairFactor { PF_MASS_INV_CUBE = 0, PF_INV_DISTANCE = 1, PF_INV_DISTANCE_FIX96 = 2 };
+
+__global__ void __launch_bounds__(256)
+    pair_factor_kernel(int kind, int64_t n, const double* __restrict__ in, double* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const double* a = in + i * (kind == PF_MASS_INV_CUBE ? 5 : kind == PF_INV_DISTANCE ? 4 : 8);
+  double got;
+  int Ee;
+  uint64_t W;
+  bool ok = emu::align_eps2(a[kind == PF_INV_DISTANCE_FIX96 ? 6 : 3], Ee, W);
+  if (kind == PF_MASS_INV_CUBE) {
+    ok = ok && emu::mass_inv_cube(a[4], a[0], a[1], a[2], Ee, W, got);
+  } else if (kind == PF_INV_DISTANCE) {
+    ok = ok && emu::inv_distance(a[0], a[1], a[2], Ee, W, got);
+  } else {
+    const int E = (int)a[7], room = W ? E - (Ee - 1023) : 1 << 20;
+    emu::Fix96 x[3], y[3];
+    for (int k = 0; k < 3; k++) {
+      x[k] = emu::to_fix96(a[k], E);
+      y[k] = emu::to_fix96(a[3 + k], E);
+    }
+    ok = ok && room >= 0 && emu::inv_distance_fix96(x, y, E, room, W, got);
+  }
+  out[i] = ok ? got : nan("");
+}
+
 // The mixed direct sum's pair arithmetic with every operand in registers: per pair 3
 // subtractions, 3 FMAs for r^2 + eps^2, one MUFU rsqrt, 3 multiplies and 3 FMAs into
 // the accumulators (12 FMA-pipe instructions and one MUFU; EQ, the equal-mass loop: 2
@@ -286,6 +316,19 @@ extern "C" int gh_check_inv_cube(int64_t n, uint64_t seed, long long* wrong_fall
   GH_CUDA_TRY(cudaStreamSynchronize(st));
   wrong_fallback[0] = (long long)h[0];
   wrong_fallback[1] = (long long)h[1];
+  return GH_OK;
+}
+
+extern "C" int gh_check_pair_factor(int kind, int64_t n, const double* in, double* out, void* stream) {
+  using namespace gh;
+  clear_error();
+  if (kind < PF_MASS_INV_CUBE || kind > PF_INV_DISTANCE_FIX96)
+    return set_error(GH_ERR_ARG, "pair factor: unknown kind %d", kind);
+  if (n < 0 || n > (1LL << 31)) return set_error(GH_ERR_ARG, "pair factor: bad count");
+  if (n == 0) return GH_OK;
+  if (!in || !out) return set_error(GH_ERR_ARG, "null buffer");
+  pair_factor_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(kind, n, in, out);
+  GH_LAUNCH_CHECK();
   return GH_OK;
 }
 

@@ -245,6 +245,14 @@ int gh_measure_l2_read(double* bytes_per_s, void* stream);
  * native path. */
 int gh_check_inv_cube(int64_t n, uint64_t seed, long long* wrong_fallback, void* stream);
 
+/* The pair factors that the FP64 tree walk and the potential form in fixed point, as the
+ * current device gives them, for n pairs (no counterpart in the reference): kind 0
+ * m s^(-3/2) of (d[3], eps^2, m), 1 s^(-1/2) of (d[3], eps^2), 2 s^(-1/2) of 96-bit
+ * fixed-point positions (a[3], b[3], eps^2, E), every |coordinate| below 2^E; s = |d|^2 +
+ * eps^2.  in (n rows of 5, 4 or 8 doubles) and out (n) are device buffers; out is NaN where
+ * a factor is refused and FP64 operations take its place.  Stream-ordered. */
+int gh_check_pair_factor(int kind, int64_t n, const double* in, double* out, void* stream);
+
 /* Builds the octree of (pos, mass) (device buffers) and checks its invariants (no
  * counterpart in the reference, whose pointer tree has none to check): out holds 9
  * entries, out[0] the number of cells, out[1] the leaves (np when the tree is whole),
