@@ -1432,6 +1432,7 @@ __global__ void __launch_bounds__(TW_THREADS, TW_MINB)
 // Workspace and host driver
 // ---------------------------------------------------------------------------
 struct TreeWS {
+  int num_sms = 0;  // of its device
   Buffer part, root, keys, keys_tmp, idx, idx_tmp, rs, lp, cnt, depth, base, scan, flags;
   Buffer nA, nC, nM, fxl, fxt, xh[2];
   Buffer wpart, wcount;       // split walks: partial sums, finished segments per group
@@ -1450,6 +1451,15 @@ struct TreeWS {
 };
 static TreeWS g_tree[64];
 static std::recursive_mutex g_tree_mu;
+
+// The current device's workspace (under g_tree_mu).
+static int tree_workspace(TreeWS** ws) {
+  DeviceInfo di;
+  GH_TRY(device_info(&di));
+  *ws = &g_tree[di.device];
+  (*ws)->num_sms = di.num_sms;
+  return GH_OK;
+}
 
 static NodeArrays node_arrays(TreeWS& ws) {
   NodeArrays na;
@@ -1472,7 +1482,6 @@ struct BuiltTree {
 // cost exceeds what the coherent warps save).
 constexpr int64_t TGT_SORT_MIN = 8192;
 
-constexpr int64_t KEYS_WIDE = 4 * 152 * 256;
 
 static int bad_input() {
   return set_error(GH_ERR_ARG,
@@ -1604,7 +1613,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
     uint32_t* itmp = (uint32_t*)ws.idx_tmp.ptr;
     int* flags = (int*)ws.flags.ptr;
     GH_CUDA_TRY(cudaMemsetAsync(flags, 0, 8 * sizeof(int), st));
-    if (n >= KEYS_WIDE)
+    if (n >= 4LL * 256 * ws.num_sms)  // four blocks of 256 per SM (see keys_kernel)
       keys_kernel<1024><<<(unsigned)((n + 1023) / 1024), 1024, 0, st>>>(pos, n, root, words, keys, idx);
     else
       keys_kernel<256><<<gn, 256, 0, st>>>(pos, n, root, words, keys, idx);
@@ -1704,8 +1713,9 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
     nodes_kernel<<<gn, T, 0, st>>>(n, lp, dep, bs, perm, pos, mass, na, nnodes, (int*)ws.list.ptr, openers, cells,
                                    (int*)ws.flags.ptr + 6);
     GH_LAUNCH_CHECK();
-    cell_centres_kernel<<<gn < 4 * 152 ? gn : 4 * 152, T, 0, st>>>(keys, words, n, lp, dep, bs, root, na,
-                                                                  (const int*)ws.list.ptr, openers);
+    const unsigned resident = 4u * (unsigned)ws.num_sms;
+    cell_centres_kernel<<<gn < resident ? gn : resident, T, 0, st>>>(keys, words, n, lp, dep, bs, root, na,
+                                                                    (const int*)ws.list.ptr, openers);
     GH_LAUNCH_CHECK();
     if (ncells > 0) {
       cells_kernel<<<(unsigned)((ncells + T - 1) / T), T, 0, st>>>(keys, words, n, lp, bs, root, na, nnodes, cells,
@@ -1875,9 +1885,9 @@ int tree_force(const double* pos, const double* mass, int64_t np, const double* 
     return GH_OK;
   }
   std::lock_guard<std::recursive_mutex> lk(g_tree_mu);
-  DeviceInfo di;
-  GH_TRY(device_info(&di));
-  TreeWS& ws = g_tree[di.device];
+  TreeWS* w = nullptr;
+  GH_TRY(tree_workspace(&w));
+  TreeWS& ws = *w;
   EpiStore epi{acc};
   for (bool again = true; again;) {
     BuiltTree bt;
@@ -1895,9 +1905,9 @@ int tree_run(double* x, double* v, const double* mass, int64_t np, int64_t nstep
              double theta, int precision, double* hist_x, double* hist_v, int64_t stride, cudaStream_t st) {
   GH_TRY(check_tree_args(np, 0, eps, precision));
   std::lock_guard<std::recursive_mutex> lk(g_tree_mu);
-  DeviceInfo di;
-  GH_TRY(device_info(&di));
-  TreeWS& ws = g_tree[di.device];
+  TreeWS* w = nullptr;
+  GH_TRY(tree_workspace(&w));
+  TreeWS& ws = *w;
   GH_TRY(ensure(ws.xh[0], (size_t)np * 3 * sizeof(double)));
   GH_TRY(ensure(ws.xh[1], (size_t)np * 3 * sizeof(double)));
   GH_TRY(drift_prepare_f64(x, v, np, dt, (double*)ws.xh[0].ptr, st));
@@ -1994,7 +2004,9 @@ extern "C" int gh_tree_validate(const double* pos, const double* mass, int64_t n
   std::lock_guard<std::recursive_mutex> lk(g_tree_mu);
   DeviceInfo di;
   GH_TRY(device_info(&di));
-  TreeWS& ws = g_tree[di.device];
+  TreeWS* w = nullptr;
+  GH_TRY(tree_workspace(&w));
+  TreeWS& ws = *w;
   BuiltTree bt;
   GH_TRY(tree_build(ws, pos, mass, np, eps, st, &bt));
   static Buffer counts[64];
