@@ -1,7 +1,7 @@
 """Autotuner for the tile shape of the mixed-precision direct-sum kernel.
 
 The library compiles ``gh_direct_num_shapes()`` tile shapes of the mixed kernel
-(packed f32x2 and scalar FP32 pair loops, 128-512 threads, 2-8 targets per thread)
+(packed f32x2 and scalar FP32 pair loops, 64-512 threads, 2-8 targets per thread)
 and picks one by size from a built-in table.  ``tune_direct`` times every shape on
 seeded Plummer spheres of the given sizes, for a force and for a fused leapfrog step,
 on the current GPU, and installs the winners as rules in the library

@@ -332,8 +332,8 @@ __global__ void vjp_reduce_mixed_kernel(const float2* __restrict__ part, int spl
 // source's sum in shared memory, a private copy per warp.  The partial sums of rows (part_i)
 // and columns (part_j) are added in a fixed order.
 // The differences come from 96-bit fixed-point positions and the inverse distance from
-// 64-bit fixed point (f64emu.cuh), about 150 instructions per unordered pair and warp (54
-// cycles of an SM as measured, ALU 71 % busy) with two DFMAs on the FP64 pipe (34 of the
+// 64-bit fixed point (f64emu.cuh), about 155 instructions per unordered pair and warp (54
+// cycles of an SM as measured, ALU 71 % busy) with two DFMAs on the FP64 pipe (32 of the
 // cycles).  With FP64 differences it took 94 cycles, and the one-sided sum in FP64 296 (three
 // differences, three DFMAs of the squared distance, a comparison, a DFMA, each twice).
 // N = 65,536: 62.9 -> 20.0 -> 11.7 ms; 8192: 996 -> 364 -> 225 us; 1000: 74 -> 70 -> 56 -> 27
@@ -582,7 +582,10 @@ struct AdjWS {
 static AdjWS g_adj[64];
 static std::mutex g_adj_mu;
 
-constexpr size_t PAIR_SCRATCH = 256u << 20;  // bytes of column sums held at once, at most
+// Bytes of column sums held at once, at most; kept for the life of the process, as every
+// workspace (with the rows' sums, some 40 MB, from 92,673 particles on for the potential, 46,337
+// for the FP64 VJP).
+constexpr size_t PAIR_SCRATCH = 256u << 20;
 
 // How an unordered-pair sum of `comps` values per particle is laid out.
 struct PairPlan {

@@ -208,8 +208,9 @@ GH_EMU_HD bool inv_cube_rn(double s, double& out) {
   return inv_cube_core(E, (bits & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull, out);
 }
 
-// s^(-3/2) of a rounded s within about half an ulp (not correctly rounded; the tree walk
-// takes mass_inv_cube below, which starts from the differences); false outside [2^-577, 2^602).
+// s^(-3/2) of a rounded s within about half an ulp (not correctly rounded); false outside
+// [2^-577, 2^602).  No kernel takes this or rsqrt1 any more (the tree walk and the potential
+// start from the differences, below); the host check holds rsqrt_powers to the same bounds.
 GH_EMU_HD bool rsqrt_cube(double s, double& out) {
   const uint64_t bits = dbits(s);
   const int E = (int)(bits >> 52);
@@ -232,8 +233,7 @@ GH_EMU_HD bool rsqrt_cube(double s, double& out) {
   return true;
 }
 
-// s^(-1/2) within about half an ulp (the FP64 potential); false outside
-// [2^-577, 2^602).
+// s^(-1/2) within about half an ulp; false outside [2^-577, 2^602).
 GH_EMU_HD bool rsqrt1(double s, double& out) {
   const uint64_t bits = dbits(s);
   const int E = (int)(bits >> 52);
@@ -271,7 +271,8 @@ GH_EMU_HD bool rsqrt_powers(double s, double& inv1, double& inv3) {
 #endif
   const uint64_t T2 = Y2sq << l2, T3 = Y3 << l3;  // in [2^63, 2^64)
   const uint64_t m2 = (T2 >> 11) + ((T2 >> 10) & 1), m3 = (T3 >> 11) + ((T3 >> 10) & 1);
-  // s^-1 = y^2 2^(-52 - p) = m2 2^(11 - 62 - l2 - 52 - p); s^(-3/2) as in rsqrt_cube
+  // s^-1 = y^2 2^(-52 - p) = m2 2^(11 - 62 - l2 - 52 - p),
+  // s^(-3/2) = y^3 2^(-3 (26 + p/2)) = m3 2^(11 - 62 - l3 - 78 - 3p/2)
   inv1 = bitsd(((uint64_t)(-103 - l2 - p + 1074) << 52) + m2);
   inv3 = bitsd(((uint64_t)(-129 - l3 - 3 * (p / 2) + 1074) << 52) + m3);
   return true;
@@ -389,12 +390,11 @@ GH_EMU_HD bool pair_inv_cube_rn(double dx, double dy, double dz, int eps2_E, uin
 }
 
 // ---------------------------------------------------------------------------
-// m s^(-3/2) with s = dx^2 + dy^2 + dz^2 + eps^2, all in 64-bit fixed point and rounded
-// once (the tree walk's FP64 interactions): the differences are aligned at the largest
+// Powers of s = dx^2 + dy^2 + dz^2 + eps^2 in 64-bit fixed point, rounded once (the tree
+// walk's FP64 interactions, the potential): the differences are aligned at the largest
 // exponent e (|d| 2^(62-e) as integers), squared to their top 64 bits and summed, so
 // s = S 2^(2e-60) with S to about 2^-58 of s and an exponent that is even as the root
-// wants it; one residual h = 1 - n y0^2 of the FP32 seed, |h| < 2^-20, then
-// s^(-3/2) = y0^3 (1 + 3/2 h + 15/8 h^2), whose first omitted term is below 2^-58.
+// wants it; then one residual h = 1 - n y0^2 of the FP32 seed, |h| < 2^-20, and a series in h.
 
 GH_EMU_HD int clz64(uint64_t v) {
 #ifdef __CUDA_ARCH__
@@ -509,7 +509,8 @@ GH_EMU_HD uint64_t scale_up(uint32_t A, int64_t C) {
   return (((uint64_t)A << 32) | (uint32_t)(((uint64_t)A * cl) >> 32)) + (uint64_t)((int64_t)(int32_t)A * ch);
 }
 
-// 1/sqrt(s), s = n 4^e, n = N10 2^-62, rounded once; false when the seed check fails.
+// 1/sqrt(s), s = n 4^e, n = N10 2^-62 in [1, 4), rounded once; false when the seed check of
+// host builds fails (rsqrt_seed_residual).
 GH_EMU_HD bool inv_root_rn(uint64_t N10, int e, double& out) {
   uint64_t Y0sq;
   uint32_t Y0;
@@ -606,6 +607,8 @@ GH_EMU_HD bool inv_distance_fix96(const Fix96* a, const Fix96* b, int E, int roo
   return ((S >> 60) != 0) & inv_root_rn(big ? S : S << 2, E - sh + big, out);
 }
 
+// m s^(-3/2), rounded once: s^(-3/2) = y0^3 (1 + 3/2 h + 15/8 h^2), whose first omitted term is
+// below 2^-58.  False outside the range of aligned_norm2 and for |m| outside [2^-500, 2^501).
 GH_EMU_HD bool mass_inv_cube(double m, double dx, double dy, double dz, int Ee, uint64_t W, double& out) {
   uint64_t N10, Y0sq;
   uint32_t Y0;

@@ -257,7 +257,7 @@ __device__ __forceinline__ void warp_append(bool need, int64_t i, int* __restric
   if (need) list[base + __popc(mask & lane_mask_lt())] = (int)i;
 }
 
-// Fast keys where the decisions are provably the recurrence's (see root_kernel); the
+// Fast keys where the decisions are provably the recurrence's (see root_write); the
 // block's other particles (about 2 %) then take the reference's recurrence
 // (gravoct_calc_subnode, _jbgrav.c:441-462), compacted so that it runs on full warps: it
 // is a chain of FP64 additions, each 20 cycles of the SM for a warp however many of its
@@ -1000,7 +1000,7 @@ __device__ __forceinline__ double rsqrt_f64(double s) {
 
 // Mixed: accepted cells interact in FP32: the hi/lo split offset of the cell's
 // centre (keeps ~2^-48 of |x|) plus the FP32 offset of its centre of mass; partial
-// sums folded into a two-sum (hi, lo) accumulator every 32 interactions.  Otherwise
+// sums folded into a two-sum (hi, lo) accumulator every TW_FOLD warp steps.  Otherwise
 // FP64 with the factor from fixed point (f64emu.cuh).
 // The opening decisions are the same exact ones in both forms.
 constexpr int TW_FOLD = 32;
@@ -1013,7 +1013,7 @@ constexpr int TW_FQ_ROUND = 28;
 static_assert((TW_FQ & (TW_FQ - 1)) == 0, "the FIFO index wraps with a mask");
 
 // Softening as the fixed-point interaction wants it (f64emu.cuh); ok = false keeps every
-// interaction on the FP64 operations. 
+// interaction on the FP64 operations.
 struct WalkEps {
   double eps2;
   uint64_t W;
@@ -1024,9 +1024,10 @@ struct WalkEps {
 // One FP64 interaction: the cell's monopole (nM) times s^(-3/2), from the differences to
 // the rounded factor in 64-bit fixed point; FP64 operations outside that form's range.
 // Bound by the FP64 pipe, which a warp's DFMA holds for 17 cycles of the SM and a DADD
-// or DMUL for 20 (measured): three differences and three sums are left on it, 111 of the
-// 106-cycle round at N = 1M (idle lanes are skipped), where s and its factor took four
-// more.  The fixed-point part is about 190 integer instructions (issue 58 % busy).
+// or DMUL for 20 (measured): three differences and three sums are left on it, busy for 96 of
+// the 109 cycles that a round takes at N = 1M (29 of 32 lanes hold an interaction), where s
+// and its factor took four more.  With the walk's steps and the fixed-point factor a round is
+// 273 instructions (issue 63 % busy).
 // Force at N = 1M Hernquist + disk: theta 0.7 29.0 -> 18.5 ms, theta 0.5 71.6 -> 44.9;
 // the differences as FMAs by an opaque 1.0 (17 cycles instead of 20): 18.8.
 // A zero mass has no place in the fixed-point factor, which would send its whole round to
@@ -1438,7 +1439,7 @@ struct TreeWS {
   Buffer wpart, wcount;       // split walks: partial sums, finished segments per group
   size_t wcount_zeroed = 0;
   Buffer tkeys, tkeys_tmp, tidx, tidx_tmp, trs;  // target points' walk order
-  Buffer list;                // particle lists: key fallbacks, then cell openers
+  Buffer list;                // particles that open internal cells
   Buffer cells;               // (internal cell, opener) pairs
   int* host_flags = nullptr;  // pinned: the 8 device flags, nnodes, the root's non-finite flag; [10..11] small build
   cudaEvent_t small_built = nullptr;
@@ -1481,7 +1482,6 @@ struct BuiltTree {
 // Target points are walked in key order from this many on (below, the sort's fixed
 // cost exceeds what the coherent warps save).
 constexpr int64_t TGT_SORT_MIN = 8192;
-
 
 static int bad_input() {
   return set_error(GH_ERR_ARG,
@@ -1592,7 +1592,7 @@ static int tree_build(TreeWS& ws, const double* pos, const double* mass, int64_t
   GH_TRY(ensure(ws.depth, n * sizeof(int)));
   GH_TRY(ensure(ws.base, (n + 1) * sizeof(int)));
   GH_TRY(ensure(ws.scan, scan_scratch_ints(n) * sizeof(int)));
-  // flags: [0] full-key tie, [1] deepest level, [2] long run, [3] key fallbacks, [4] cell openers,
+  // flags: [0] full-key tie, [1] deepest level, [2] long run, [4] cell openers,
   // [5] a bounded wait in the sort gave up, [6] internal cells listed
   GH_TRY(ensure(ws.flags, 8 * sizeof(int)));
   GH_TRY(ensure(ws.list, n * sizeof(int)));
@@ -1743,11 +1743,15 @@ static Buffer g_stats[64];
 // about 2 % more steps per doubling (the ancestors of each segment's first cell).
 // All in all 14,000 warps and n / 5 more were fastest (a larger tree has more steps to
 // share), at most 64 per group of particles, 128 of sorted points and 256 of unsorted ones.
-// Less than 12 for each of many groups is worse than two, and 3/8 of a million targets
-// fill the GPU unsplit.  Force, unsplit -> split, theta 0.7: N = 500 Plummer 302 -> 96 us,
+// Where that is less than 12 for each of many groups, two, whose ranges meet at the group's
+// own place: with Hernquist + disk, 11 / two (us), theta 0.7 and 0.5: N = 75,000 1651 / 1532
+// and 3103 / 3119, 90,113 1916 / 1920 and 3795 / 4026, 110,000 2158 / 2222 and 4330 / 4981,
+// 131,072 2563 / 2361 and 5145 / 5095, 200,000 3669 / 3513 and 7932 / 8092; 3 to 8 are worse
+// than the better of the two.  So neither wins throughout, and the line is where theta 0.7
+// changes sides for good.  3/8 of a million targets fill the GPU unsplit (393,217: 6833 us, two
+// 6704; 1,048,576 18.7 ms, two 19.1).  Force, unsplit -> split, theta 0.7: N = 500 Plummer 302 -> 96 us,
 // 2000 577 -> 131, 8000 840 -> 303; Hernquist + disk 16,384 1304 -> 575, 30,000 1541 ->
-// 842, 60,013 1835 -> 1375, 131,072 2580 -> 2540, 262,144 4847 -> 4590; at 1,048,576 two
-// warps would cost 18.7 -> 19.1 ms.  Points in a 250,000-particle system, theta 0.5: 100
+// 842, 60,013 1726 -> 1372, 131,072 2392 -> 2359, 262,144 4638 -> 4477.  Points in a 250,000-particle system, theta 0.5: 100
 // unsorted 17.6 -> 0.85 ms, 8100 16.9 -> 2.9, 10,000 sorted 7.0 -> 1.8, 30,011 6.0 -> 2.8,
 // 100,000 6.3 -> 5.5.
 static int walk_segments(int64_t groups, int64_t n, int cap) {

@@ -13,7 +13,10 @@
  * before returning.  "_dev" entry points take device pointers and a cudaStream_t
  * (passed as void*, NULL = legacy default stream) and are stream-ordered: they return
  * once the work is enqueued.  The library keeps one grow-only device workspace per
- * device; calls that use it must not run concurrently on different streams.
+ * device; calls that use it must not run concurrently on different streams.  It is kept
+ * for the life of the process: a few hundred bytes per particle for the tree, and up to
+ * about 300 MB (256 of column sums, the rows' sums beside them) for the potential and the
+ * FP64 VJP, which sum each unordered pair once.
  */
 #ifndef GRAVHOPPER_GB300_H
 #define GRAVHOPPER_GB300_H
