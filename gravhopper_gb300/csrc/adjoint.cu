@@ -336,7 +336,7 @@ __global__ void vjp_reduce_mixed_kernel(const float2* __restrict__ part, int spl
 // cycles of an SM as measured, ALU 71 % busy) with two DFMAs on the FP64 pipe (32 of the
 // cycles).  With FP64 differences it took 94 cycles, and the one-sided sum in FP64 296 (three
 // differences, three DFMAs of the squared distance, a comparison, a DFMA, each twice).
-// N = 65,536: 62.9 -> 20.0 -> 11.7 ms; 8192: 996 -> 364 -> 225 us; 1000: 74 -> 70 -> 56 -> 27
+// N = 65,536: 62.9 -> 20.0 -> 11.7 ms; 8192: 996 -> 364 -> 225 us; 1000: 74 -> 70 -> 56 -> 28
 // in shares.
 // Two or four targets per thread: the same from N = 30,000 on, slower below (fewer CTAs).
 // ---------------------------------------------------------------------------
@@ -468,28 +468,54 @@ __global__ void __launch_bounds__(AJ_THREADS)
 }
 
 // Adds the sums of rows row0 .. row0 + rows - 1: a particle's own row, split by split, then
-// the rows that met its block as a column, in row order.  C sums per particle, one per
-// blockIdx.y: the first of them to out (stride C < 4 ? C : 3), a fourth to out4.
-template <int C>
+// the rows that met its block as a column, in row order; the shares of a pair of blocks among
+// themselves first (added one by one to the whole sum they doubled its error: 3e-16 against
+// 1.4e-16 in the potential of 1500 particles).  C sums per particle, one per blockIdx.y: the
+// first of them to out (stride C < 4 ? C : 3), a fourth to out4.
+template <int C, int PARTS>
 __global__ void pairs_reduce_kernel(const double* __restrict__ part_i, const double* __restrict__ part_j, int64_t n,
-                                    int nblocks, int row0, int rows, int parts, int splits,
-                                    double* __restrict__ out, double* __restrict__ out4) {
+                                    int nblocks, int row0, int rows, int splits, double* __restrict__ out,
+                                    double* __restrict__ out4) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int c = blockIdx.y;
   double* to = c == 3 ? out4 + k : out + k * (C < 4 ? C : 3) + c;
   const int J = (int)(k / AJ_THREADS), o = (int)(k - (int64_t)J * AJ_THREADS) + c * AJ_THREADS, dmax = nblocks / 2;
   double a = row0 ? *to : 0.0;
-  if (J >= row0 && J < row0 + rows)
-#pragma unroll 8
-    for (int s = 0; s < splits; s++) a += part_i[((int64_t)(J - row0) * splits + s) * C * AJ_THREADS + o];
+  if (J >= row0 && J < row0 + rows) {
+    const double* own = part_i + (int64_t)(J - row0) * splits * C * AJ_THREADS + o;
+    int s = 0;
+    for (; s + PARTS <= splits; s += PARTS) {
+      double t = own[(int64_t)s * C * AJ_THREADS];
+#pragma unroll
+      for (int q = 1; q < PARTS; q++) t += own[(int64_t)(s + q) * C * AJ_THREADS];
+      a += t;
+    }
+    for (; s < splits; s++) a += own[(int64_t)s * C * AJ_THREADS];
+  }
   for (int r = 0; r < rows; r++) {
     const int I = row0 + r;
     const int d = J >= I ? J - I : J - I + nblocks;
     if (d < 1 || d > dmax || (2 * d == nblocks && I >= nblocks / 2)) continue;
-    for (int p = 0; p < parts; p++) a += part_j[(((int64_t)r * dmax + d - 1) * parts + p) * C * AJ_THREADS + o];
+    const double* col = part_j + ((int64_t)r * dmax + d - 1) * PARTS * C * AJ_THREADS + o;
+    double t = *col;
+#pragma unroll
+    for (int q = 1; q < PARTS; q++) t += col[(int64_t)q * C * AJ_THREADS];
+    a += t;
   }
   *to = a;
+}
+
+template <int C>
+static int launch_pairs_reduce(const double* part_i, const double* part_j, int64_t n, int nblocks, int row0, int rows,
+                               int parts, int splits, double* out, double* out4, int sums, cudaStream_t st) {
+  const auto kernel = parts == 1   ? pairs_reduce_kernel<C, 1>
+                      : parts == 8 ? pairs_reduce_kernel<C, 8>
+                                   : pairs_reduce_kernel<C, 32>;
+  kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)sums), 256, 0, st>>>(part_i, part_j, n, nblocks, row0, rows, splits,
+                                                                           out, out4);
+  GH_LAUNCH_CHECK();
+  return GH_OK;
 }
 
 // Mass-weighted centre for the FP32 sources, in 256 chains (particles t, t + 256, ...) of
@@ -621,8 +647,9 @@ static int plan_pairs(AdjWS& ws, int64_t n, int comps, int parts, int num_sms, P
 // A pair of blocks is a chain of 128 pairs per lane, some 200 us in the VJP and 45 in the
 // potential; shares of it where the pairs of blocks are few.  VJP: N = 100 32 shares 167 -> 15
 // us, 1000 8 shares 227 -> 76, 6000 1329 -> 1277; more blocks lose (16,384 8981 -> 9220).
-// Potential: N = 30 31 -> 17 us (of one block, which finds its own largest coordinate), 129 50
-// -> 23, 1000 55 -> 27, 3000 74 -> 68; more blocks lose (4000 88 -> 96).
+// Potential (device time): N = 30 27 -> 7 us (of one block, which finds its own largest
+// coordinate), 130 46 -> 19, 1000 50 -> 23, 3000 69 -> 61; more blocks lose (4000 83 -> 91).
+// (pairs_reduce_kernel is made for 1, 8 and 32.)
 static int pair_shares(int64_t n, bool vjp) {
   const int64_t nb = (n + AJ_THREADS - 1) / AJ_THREADS, meets = nb * (nb / 2 + 1);
   return meets < 8 ? 32 : (meets < (vjp ? 1200 : 320) ? 8 : 1);
@@ -652,10 +679,8 @@ int direct_vjp(const double* pos, const double* mass, int64_t n, double eps, con
           (double*)ws.part_j.ptr);
       prof_end(st);
       GH_LAUNCH_CHECK();
-      pairs_reduce_kernel<4><<<dim3(rb, gmass ? 4 : 3), 256, 0, st>>>(
-          (const double*)ws.part.ptr, (const double*)ws.part_j.ptr, n, pp.nblocks, row0, here, pp.parts, (int)pp.splits, gpos,
-          gmass);
-      GH_LAUNCH_CHECK();
+      GH_TRY(launch_pairs_reduce<4>((const double*)ws.part.ptr, (const double*)ws.part_j.ptr, n, pp.nblocks, row0, here,
+                                    pp.parts, (int)pp.splits, gpos, gmass, gmass ? 4 : 3, st));
     }
     return GH_OK;
   }
@@ -891,11 +916,8 @@ int potential(const double* pos, const double* mass, int64_t n, double eps, doub
     kernel<<<grid, AJ_THREADS, 0, st>>>(pos, mass, n, eps * eps, largest, pp.nblocks, row0, pp.parts, pp.len,
                                         (double*)ws.part.ptr, (double*)ws.part_j.ptr);
     GH_LAUNCH_CHECK();
-    pairs_reduce_kernel<1><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const double*)ws.part.ptr,
-                                                                       (const double*)ws.part_j.ptr, n, pp.nblocks,
-                                                                       row0, here, pp.parts, (int)pp.splits, phi,
-                                                                       nullptr);
-    GH_LAUNCH_CHECK();
+    GH_TRY(launch_pairs_reduce<1>((const double*)ws.part.ptr, (const double*)ws.part_j.ptr, n, pp.nblocks, row0, here,
+                                  pp.parts, (int)pp.splits, phi, nullptr, 1, st));
   }
   return GH_OK;
 }
