@@ -1021,6 +1021,20 @@ struct WalkEps {
   bool ok;
 };
 
+// m s^(-3/2) where the fixed-point factor does not take the pair: FP64 operations, 0 for
+// s = 0; but a zero mass, which has no place in that factor either, is its own (as FP64 it
+// cost its whole round: 300,000 particles, a fifth massless, 6.30 -> 4.42 ms, none 3.82).  A
+// call: inline, it cost the rounds that do not take it up to 0.5 % (60,013 1377 -> 1365 us).
+template <bool GUARD>
+__device__ __noinline__ double walk_factor_rare(double m, double dx, double dy, double dz, double eps2, int Ee, bool ok) {
+  double f;
+  if (ok && emu::zero_mass_inv_cube(m, dx, dy, dz, Ee, f)) return f;
+  const double s = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
+  if (GUARD && s == 0.0) return 0.0;
+  const double y = rsqrt_f64(s);
+  return m * (y * (y * y));
+}
+
 // One FP64 interaction: the cell's monopole (nM) times s^(-3/2), from the differences to
 // the rounded factor in 64-bit fixed point; FP64 operations outside that form's range.
 // Bound by the FP64 pipe, which a warp's DFMA holds for 17 cycles of the SM and a DADD
@@ -1030,22 +1044,14 @@ struct WalkEps {
 // 273 instructions (issue 63 % busy).
 // Force at N = 1M Hernquist + disk: theta 0.7 29.0 -> 18.5 ms, theta 0.5 71.6 -> 44.9;
 // the differences as FMAs by an opaque 1.0 (17 cycles instead of 20): 18.8.
-// A zero mass has no place in the fixed-point factor, which would send its whole round to
-// the FP64 operations; its factor is the mass itself (300,000 particles, a fifth massless:
-// 6.30 -> 4.42 ms, none 3.82).
 template <bool GUARD>
 __device__ __forceinline__ void walk_interact_f64(const dvec4* __restrict__ nM, int node, double p0, double p1,
                                                   double p2, const WalkEps& E, double& ax, double& ay, double& az) {
   const dvec4 M = nM[node];
   const double dx = M.x - p0, dy = M.y - p1, dz = M.z - p2;
   double f;
-  if (!(E.ok && (emu::mass_inv_cube(M.w, dx, dy, dz, E.E, E.W, f) ||
-                 emu::zero_mass_inv_cube(M.w, dx, dy, dz, E.E, f)))) {
-    const double s = fma(dx, dx, fma(dy, dy, fma(dz, dz, E.eps2)));
-    if (GUARD && s == 0.0) return;
-    const double y = rsqrt_f64(s);
-    f = M.w * (y * (y * y));
-  }
+  if (!(E.ok && emu::mass_inv_cube(M.w, dx, dy, dz, E.E, E.W, f)))
+    f = walk_factor_rare<GUARD>(M.w, dx, dy, dz, E.eps2, E.E, E.ok);
   ax = fma(f, dx, ax);
   ay = fma(f, dy, ay);
   az = fma(f, dz, az);
