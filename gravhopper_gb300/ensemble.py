@@ -27,7 +27,7 @@ class Ensemble:
         self.device = device or torch.device("cuda", torch.cuda.current_device())
         ns = np.array([len(s["mass"]) for s in systems], dtype=np.int64)
         for n, s in zip(ns, systems):
-            if np.shape(s["mass"]) != (n,) or np.shape(s["pos"]) != (n, 3) or np.shape(s["vel"]) != (n, 3):
+            if [int(np.prod(np.shape(s[k]))) for k in ("pos", "vel", "mass")] != [3 * n, 3 * n, n]:
                 raise ValueError("each system needs pos and vel of shape (N,3) and mass of shape (N,)")
         self.offsets = np.concatenate([[0], np.cumsum(ns)]).astype(np.int64)
         self.eps = np.array([float(s["eps"]) for s in systems], dtype=np.float64)

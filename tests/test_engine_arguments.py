@@ -51,7 +51,7 @@ def test_ensemble_refuses_ragged_systems():
     from gravhopper_gb300.ensemble import Ensemble
     good = {"pos": f64(4, 3), "vel": f64(4, 3), "mass": f64(4), "eps": 0.1, "dt": 0.1}
     assert Ensemble([good], device="cpu").nsys == 1
-    for k, v in (("pos", f64(3, 3)), ("vel", f64(5, 3)), ("pos", f64(12)), ("mass", f64(4, 1))):
+    for k, v in (("pos", f64(3, 3)), ("vel", f64(5, 3)), ("pos", f64(4, 2)), ("mass", f64(4, 2))):
         with pytest.raises(ValueError):
             Ensemble([good, dict(good, **{k: v})], device="cpu")
 
